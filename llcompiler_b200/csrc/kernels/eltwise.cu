@@ -7,67 +7,12 @@
 #include <vector>
 
 #include "common.cuh"
+#include "eltwise_prog.cuh"
 
 namespace llc {
 namespace {
 
-constexpr int kMaxInstr = 48;
-constexpr int kMaxRank = 6;
-constexpr int kMaxIn = 8;
-
-enum EltOp : int {
-  E_LD = 0, E_IMM, E_ADD, E_SUB, E_MUL, E_DIV, E_MAX, E_MIN, E_POW, E_RELU, E_ABS, E_SQRT, E_RSQRT, E_EXP, E_GELU, E_TANH,
-  E_ERF, E_SIGMOID, E_NEG, E_CAST, E_TRUNC, E_TF32LO, E_WHERE, E_EQ, E_NE, E_GE, E_GT, E_LE, E_LT
-};
-
-struct EltProgram {
-  int n;
-  unsigned char op[kMaxInstr], a[kMaxInstr], b[kMaxInstr], c[kMaxInstr];
-  float imm[kMaxInstr];
-};
-
-struct EltArgs {
-  void* out; int odt; int rank; int nin;
-  long long shape[kMaxRank], ostr[kMaxRank];
-  const void* in[kMaxIn]; int idt[kMaxIn]; long long istr[kMaxIn][kMaxRank];
-  long long total;      // number of output elements
-  int innerVec;         // elements handled per thread along the innermost dim (1 or 4)
-  EltProgram prog;
-};
-
-__device__ __forceinline__ float evalOp(int op, float x, float y, float z, float imm) {
-  switch (op) {
-    case E_IMM: return imm;
-    case E_ADD: return x + y;
-    case E_SUB: return x - y;
-    case E_MUL: return x * y;
-    case E_DIV: return x / y;
-    case E_MAX: return fmaxf(x, y);
-    case E_MIN: return fminf(x, y);
-    case E_POW: return powf(x, y);
-    case E_RELU: return fmaxf(x, 0.f);
-    case E_ABS: return fabsf(x);
-    case E_SQRT: return sqrtf(x);
-    case E_RSQRT: return rsqrtf(x);
-    case E_EXP: return expf(x);
-    case E_GELU: return geluErf(x);
-    case E_TANH: return tanhf(x);
-    case E_ERF: return erff(x);
-    case E_SIGMOID: return 1.f / (1.f + expf(-x));
-    case E_NEG: return -x;
-    case E_CAST: return x;
-    case E_TRUNC: return truncf(x);
-    case E_TF32LO: return x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);   // what a tf32 operand read drops
-    case E_WHERE: return x != 0.f ? y : z;
-    case E_EQ: return x == y ? 1.f : 0.f;
-    case E_NE: return x != y ? 1.f : 0.f;
-    case E_GE: return x >= y ? 1.f : 0.f;
-    case E_GT: return x > y ? 1.f : 0.f;
-    case E_LE: return x <= y ? 1.f : 0.f;
-    case E_LT: return x < y ? 1.f : 0.f;
-  }
-  return 0.f;
-}
+using namespace elt;
 
 // One thread produces V consecutive elements of the innermost (unit output stride) dim.
 template <int V>
@@ -151,17 +96,6 @@ __global__ void __launch_bounds__(256) eltwise_vec_kernel(const __grid_constant_
 // program in real registers (the general kernels above index their register file dynamically, which puts it in local
 // memory).  This is the path of the big memory-bound steps: layout copies, embedding sums, residual adds, casts.
 constexpr int kSmallProg = 4;
-template <typename T> __device__ __forceinline__ void load8(const T* p, float* v);
-template <> __device__ __forceinline__ void load8<float>(const float* p, float* v) {
-  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-template <> __device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16* p, float* v) {
-  const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p));
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-  for (int e = 0; e < 4; ++e) { const float2 f = __bfloat1622float2(h[e]); v[2 * e] = f.x; v[2 * e + 1] = f.y; }
-}
 __device__ __forceinline__ float pick4(const float (*r)[8], int which, int v) {
   const float lo = which & 1 ? r[1][v] : r[0][v], hi = which & 1 ? r[3][v] : r[2][v];
   return which & 2 ? hi : lo;
@@ -182,33 +116,6 @@ __device__ __forceinline__ void eltwiseSmallBody(const EltArgs& p, long long oOf
     else load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(base) + off, dst);
   };
   float o[8];
-  // the two shapes almost every large step has: one operand (a copy, a cast, one unary op) or two operands and one
-  // binary op; the op is decoded once, outside the element loop
-  const int n = p.prog.n;
-  const bool unary = (n == 1 || (n == 2 && p.prog.op[1] != E_LD && p.prog.op[1] != E_IMM && p.prog.a[1] == 0)) && p.prog.op[0] == E_LD;
-  const bool binary = n == 3 && p.prog.op[0] == E_LD && p.prog.op[1] == E_LD && p.prog.op[2] >= E_ADD && p.prog.op[2] <= E_MIN && p.prog.a[2] + p.prog.b[2] == 1;
-  if (unary) {
-    loadOperand(p.prog.a[0], o);
-    if (n == 2) {
-      const int op = p.prog.op[1];
-      if (op == E_RELU) {
-#pragma unroll
-        for (int v = 0; v < 8; ++v) o[v] = fmaxf(o[v], 0.f);
-      } else if (op != E_CAST) {
-#pragma unroll
-        for (int v = 0; v < 8; ++v) o[v] = evalOp(op, o[v], o[v], o[v], 0.f);
-      }
-    }
-  } else if (binary) {
-    float x[8], y[8];
-    loadOperand(p.prog.a[p.prog.a[2]], x); loadOperand(p.prog.a[p.prog.b[2]], y);
-    switch (p.prog.op[2]) {
-#define LLC_BIN(OP, EXPR) case OP: _Pragma("unroll") for (int v = 0; v < 8; ++v) o[v] = EXPR; break;
-      LLC_BIN(E_ADD, x[v] + y[v]) LLC_BIN(E_SUB, x[v] - y[v]) LLC_BIN(E_MUL, x[v] * y[v]) LLC_BIN(E_DIV, x[v] / y[v])
-      LLC_BIN(E_MAX, fmaxf(x[v], y[v])) LLC_BIN(E_MIN, fminf(x[v], y[v]))
-#undef LLC_BIN
-    }
-  } else {
   float r[kSmallProg][8];
 #pragma unroll
   for (int i = 0; i < kSmallProg; ++i) {
@@ -229,7 +136,6 @@ __device__ __forceinline__ void eltwiseSmallBody(const EltArgs& p, long long oOf
   }
 #pragma unroll
   for (int v = 0; v < 8; ++v) o[v] = pick4(r, p.prog.n - 1, v);
-  }
 
   if (p.odt == LLC_FLOAT32) {
     float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + oOff);
@@ -526,6 +432,19 @@ extern "C" int llc_cuda_nchw_to_nhwc(const void* x, void* out, int32_t dtype, in
   const bool f32 = dtype == LLC_FLOAT32;
   const bool aligned = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   const unsigned blocks = (unsigned)((n * hw + 255) / 256);
+  if (c_pad == c && c >= 32) {
+    // no padding: a copy whose operand runs along the pixels and whose output runs along the channels
+    EltArgs e{};
+    e.out = out; e.odt = dtype; e.rank = 3; e.nin = 1;
+    e.shape[0] = n; e.shape[1] = hw; e.shape[2] = c;
+    e.ostr[0] = hw * c; e.ostr[1] = c; e.ostr[2] = 1;
+    e.in[0] = x; e.idt[0] = dtype; e.istr[0][0] = c * hw; e.istr[0][1] = 1; e.istr[0][2] = hw;
+    e.total = n * hw * c;
+    e.prog.n = 1; e.prog.op[0] = E_LD;
+    bool taken = false;
+    const int rc = launchChain(e, st, &taken);
+    if (rc != LLC_OK || taken) return rc;
+  }
   if (aligned && f32 && c_pad == 4) nchw_to_nhwc_small_kernel<float, 4><<<blocks, 256, 0, st>>>((const float*)x, (float*)out, n, (int)c, hw);
   else if (aligned && f32 && c_pad == 8) nchw_to_nhwc_small_kernel<float, 8><<<blocks, 256, 0, st>>>((const float*)x, (float*)out, n, (int)c, hw);
   else if (aligned && !f32 && c_pad == 8) nchw_to_nhwc_small_kernel<__nv_bfloat16, 8><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)out, n, (int)c, hw);
@@ -579,6 +498,9 @@ extern "C" int llc_cuda_eltwise(const LlcEltwiseParams* q, void* stream) {
   if (r == 0) { a.shape[0] = 1; a.ostr[0] = 1; for (int k = 0; k < q->n_in; ++k) a.istr[k][0] = 0; r = 1; }
   a.rank = r; a.total = total;
   cudaStream_t st = (cudaStream_t)stream;
+  bool taken = false;
+  rc = launchChain(a, st, &taken);
+  if (rc != LLC_OK || taken) return rc;
   const long long inner = a.shape[r - 1];
   auto isVecType = [](int dt) { return dt == LLC_FLOAT32 || dt == LLC_BFLOAT16; };
   auto alignedFor = [](const void* p, int dt) { return (reinterpret_cast<uintptr_t>(p) % (dt == LLC_FLOAT32 ? 16 : 8)) == 0; };
