@@ -45,8 +45,58 @@ __device__ __forceinline__ bool mbarWait(uint64_t* bar, uint32_t parity, volatil
   return false;
 }
 
+// The same for a barrier that threads or MMAs of the other CTA of a pair arrive on: what they wrote before is visible after it.
+__device__ __forceinline__ bool mbarWaitCluster(uint64_t* bar, uint32_t parity, volatile int* abortWord) {
+  uint32_t addr = smemAddr(bar);
+  for (uint32_t i = 0; i < kSpinLimit; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
+    if (ok) return true;
+    if ((i & 255) == 255 && *abortWord) return false;
+  }
+  *abortWord = 1;
+  return false;
+}
+
 // generic-proxy writes to shared memory -> visible to the async proxy (tensor core, TMA)
 __device__ __forceinline__ void fenceProxyAsync() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// ---- CTA pairs (clusters of two) ---------------------------------------------------------------
+__device__ __forceinline__ uint32_t clusterCtaRank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+// Barrier over every thread of the cluster, with release / acquire of what was written before it.
+__device__ __forceinline__ void clusterSync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Arrives on the barrier at the same place in CTA 0 of the pair (its own CTA for CTA 0).  What the arrival hands over has
+// its own fences (tcgen05.fence for accumulators, fence.proxy.async for operand tiles); a cluster-scope release on top
+// would wait for every store of the thread (1600 cycles in the GEMM's epilogue).
+__device__ __forceinline__ void mbarArriveLeader(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .b32 a;\n\t"
+      "mapa.shared::cluster.u32 a, %0, 0;\n\t"
+      "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}"
+      ::"r"(smemAddr(bar)) : "memory");
+}
+// The shared::cluster address of the same place in the even CTA of the pair: bit 24 of a CTA's shared addresses is its rank's parity.
+__device__ __forceinline__ uint32_t leaderAddr(const void* p) { return smemAddr(p) & 0xFEFFFFFFu; }
+// Tiled / im2col loads into this CTA's shared memory whose bytes are counted by the barrier of CTA 0 of the pair.
+__device__ __forceinline__ void tmaLoadPair4d(void* smemDst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smemAddr(smemDst)), "l"((uint64_t)map), "r"(leaderAddr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+__device__ __forceinline__ void tmaLoadPairIm2col4d(void* smemDst, const CUtensorMap* map, uint64_t* bar, int c, int w, int h, int n, uint16_t offW, uint16_t offH) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.im2col.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
+      ::"r"(smemAddr(smemDst)), "l"((uint64_t)map), "r"(leaderAddr(bar)), "r"(c), "r"(w), "r"(h), "r"(n), "h"(offW), "h"(offH)
+      : "memory");
+}
 
 __device__ __forceinline__ void tmaLoad4d(void* smemDst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
   asm volatile(
@@ -77,8 +127,28 @@ __device__ __forceinline__ void bulkWaitRead() { asm volatile("cp.async.bulk.wai
 // Same, but lets the most recent store still read: with two staging slots used in turn, the slot about to be
 // rewritten belongs to the store before the last one.
 __device__ __forceinline__ void bulkWaitRead1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+__device__ __forceinline__ void bulkWaitRead3() { asm volatile("cp.async.bulk.wait_group.read 3;" ::: "memory"); }   // four slots
 __device__ __forceinline__ void prefetchTensorMap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
+}
+
+// (x0, x1) = (x0, x1) * (s0, s1) + (b0, b1), two fp32 multiply-adds in one instruction.
+__device__ __forceinline__ void fma2(float& x0, float& x1, float s0, float s1, float b0, float b1) {
+  asm("{\n\t.reg .b64 x, s, b;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 s, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "fma.rn.f32x2 x, x, s, b;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "+f"(x0), "+f"(x1) : "f"(s0), "f"(s1), "f"(b0), "f"(b1));
+}
+// geluTanhBf16 (common.cuh) of two values, the same operations on packed pairs.
+__device__ __forceinline__ void geluTanhBf16x2(float& x0, float& x1) {
+  float u0, u1, h0, h1;
+  asm("{\n\t.reg .b64 x, u, a, b, h;\n\tmov.b64 x, {%4, %5};\n\tmov.b64 a, {%6, %6};\n\tmov.b64 b, {%7, %7};\n\tmov.b64 h, {%8, %8};\n\t"
+      "mul.rn.f32x2 u, x, x;\n\tfma.rn.f32x2 u, u, a, b;\n\tmul.rn.f32x2 u, x, u;\n\tmul.rn.f32x2 h, x, h;\n\t"
+      "mov.b64 {%0, %1}, u;\n\tmov.b64 {%2, %3}, h;\n\t}"
+      : "=f"(u0), "=f"(u1), "=f"(h0), "=f"(h1) : "f"(x0), "f"(x1), "f"(0.0356774081f), "f"(0.7978845608f), "f"(0.5f));
+  asm("tanh.approx.f32 %0, %1;" : "=f"(u0) : "f"(u0));
+  asm("tanh.approx.f32 %0, %1;" : "=f"(u1) : "f"(u1));
+  fma2(h0, h1, u0, u1, h0, h1);
+  x0 = h0; x1 = h1;
 }
 
 // ---- tensor memory ------------------------------------------------------------------------------
@@ -89,6 +159,14 @@ __device__ __forceinline__ void tmemAlloc(uint32_t* slot, uint32_t cols) {
 }
 __device__ __forceinline__ void tmemDealloc(uint32_t taddr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+}
+// The same for both CTAs of a pair at once (executed by the same warp of each).
+__device__ __forceinline__ void tmemAllocPair(uint32_t* slot, uint32_t cols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(slot)), "r"(cols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmemDeallocPair(uint32_t taddr, uint32_t cols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 __device__ __forceinline__ void tcFenceBefore() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcFenceAfter() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -137,6 +215,26 @@ __device__ __forceinline__ void mmaSS(uint32_t tmemD, uint64_t descA, uint64_t d
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmemD), "l"(descA), "l"(descB), "r"(idesc), "r"(accumulate) : "memory");
   }
+}
+// One MMA over a CTA pair: M = 256, CTA r holds rows 128 r..+127 of A and of the accumulator and half r of the rows of B;
+// issued by CTA 0 with descriptors that name the same places in both CTAs.
+template <bool TF32>
+__device__ __forceinline__ void mmaPairSS(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t idesc, uint32_t accumulate) {
+  if (TF32) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmemD), "l"(descA), "l"(descB), "r"(idesc), "r"(accumulate) : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmemD), "l"(descA), "l"(descB), "r"(idesc), "r"(accumulate) : "memory");
+  }
+}
+// Arrives on the barriers at this place in both CTAs of the pair once every pair MMA issued so far has completed.
+__device__ __forceinline__ void mmaCommitPair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smemAddr(bar)), "h"((uint16_t)3) : "memory");
 }
 // Arrives on `bar` once every tcgen05.mma issued so far by this thread has completed.
 __device__ __forceinline__ void mmaCommit(uint64_t* bar) {
