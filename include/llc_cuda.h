@@ -141,6 +141,19 @@ int llc_cuda_layernorm(const void* x, const void* gamma, const void* beta, void*
 int llc_cuda_gather(const void* table, const int64_t* ids, void* out, int32_t table_dtype, int32_t out_dtype,
                     int64_t rows, int64_t d, int64_t vocab, int32_t* bad_ids, void* stream);
 
+/* out[r,:] = LayerNorm(table[ids[r],:] + add[(r / period) * add_s0 + (r % period) * add_s1 + (0..d-1)]) * gamma + beta in one
+ * pass: llc_cuda_gather, the elementwise add (rounded to the storage type, as that step stores it) and llc_cuda_layernorm
+ * where nothing else reads what is between them.  All tensors of one type, f32 or bf16.  add may be NULL.  Rows with an id outside [0, vocab) use zeros for the
+ * table row and are counted in *bad_ids when it is not NULL. */
+typedef struct LlcEmbedNormParams {
+  const void* table; const int64_t* ids; const void* add; const void* gamma; const void* beta; void* out;
+  int32_t dtype;
+  int64_t rows, d, vocab, period, add_s0, add_s1;
+  float eps;
+  int32_t* bad_ids;
+} LlcEmbedNormParams;
+int llc_cuda_embed_norm(const LlcEmbedNormParams* p, void* stream);
+
 /* x [n, c, hw] (NCHW planes) -> out [n, hw, c_pad] (NHWC pixels), channels c..c_pad-1 written as
  * zeros.  The layout change the reference expresses as llh.transpose perms [0,2,3,1] around conv
  * (src/Dialect/LLH/Transforms/TransformLayout.cpp:141-198), with the channel padding the

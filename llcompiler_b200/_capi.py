@@ -132,10 +132,15 @@ class LlcEltwiseParams(Structure):
                 ("out_strides", c_int64 * 6), ("n_in", c_int32), ("inputs", LlcEltwiseOperand * 8), ("prog", c_char_p)]
 
 
+class LlcEmbedNormParams(Structure):
+    _fields_ = [("table", c_void_p), ("ids", c_void_p), ("add", c_void_p), ("gamma", c_void_p), ("beta", c_void_p), ("out", c_void_p),
+                ("dtype", c_int32)] + [(n, c_int64) for n in ("rows", "d", "vocab", "period", "add_s0", "add_s1")] + [("eps", c_float), ("bad_ids", c_void_p)]
+
+
 EXPORTED_SYMBOLS = [
     "llc_compile", "llc_run_pass", "llc_load", "llc_load_from", "llc_loaded_from_pool", "llc_num_inputs", "llc_num_outputs", "llc_num_symbols",
     "llc_output_shape", "llc_run", "llc_profile", "llc_status", "llc_last_launch_count", "llc_arena_bytes", "llc_free", "llc_last_error",
     "llc_version", "llc_cuda_gemm", "llc_cuda_conv2d", "llc_cuda_maxpool2d", "llc_cuda_reduce",
     "llc_cuda_softmax", "llc_cuda_layernorm", "llc_cuda_gather", "llc_cuda_eltwise", "llc_cuda_status", "llc_cuda_nchw_to_nhwc", "llc_cuda_gemm_static_scratch", "llc_cuda_attention", "llc_cuda_nchw_to_nhwc_wide",
-    "llc_cuda_push_rows",
+    "llc_cuda_push_rows", "llc_cuda_embed_norm",
 ]

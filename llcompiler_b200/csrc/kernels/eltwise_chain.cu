@@ -442,7 +442,9 @@ int launchChain(const EltArgs& a, cudaStream_t st, bool* taken) {
   for (int k = 0; k < nin && rowsOk; ++k) {
     const long long s = e.istr[k][last];
     if (s == 0) continue;
-    rowsOk = s == 1 && isVecType(e.idt[k]) && alignedTo(e.in[k], 16);
+    rowsOk = s == 1;
+    if (!isVecType(e.idt[k])) continue;            // other types (an integer mask) are read element by element
+    rowsOk = rowsOk && alignedTo(e.in[k], 16);
     for (int d = 0; d < last && rowsOk; ++d) rowsOk = e.istr[k][d] % 8 == 0;
   }
   if (rowsOk) {

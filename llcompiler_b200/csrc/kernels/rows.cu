@@ -216,6 +216,138 @@ int launchLayerNormWarp(const void* x, const void* g, const void* b, void* out, 
   return LLC_OK;
 }
 
+// ---- embedding lookup + (position) add + LayerNorm ------------------------------------------------
+// The front of an encoder in one pass: table[ids[row]], rounded to its storage type like the steps it replaces after the add,
+// normalised as in layernorm_warp_kernel.  One warp per row, grid-stride; the next row's table and add vectors are in flight
+// under the current row's statistics and the id of the row after that is already there.
+// Bound: HBM writes (the table is read from L2 after its first rows).  As gather, add and LayerNorm 98304 x 768 bf16 took
+// three passes over 151 MB.
+struct EmbedNormArgs {
+  const void* table; const long long* ids; const void* add; const void* gamma; const void* beta; void* out; int* bad;
+  long long rows, vocab, period, s0, s1;        // the added row of `row` starts at (row / period) * s0 + (row % period) * s1
+  int d; float eps;
+};
+template <typename T, int NV>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32) embed_norm_kernel(const __grid_constant__ EmbedNormArgs p) {
+  constexpr int E = 16 / sizeof(T);
+  const int lane = threadIdx.x & 31, d = p.d;
+  const long long step = (long long)gridDim.x * kWarpsPerBlock;
+  long long row = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (row >= p.rows) return;
+  const T* table = reinterpret_cast<const T*>(p.table);
+  const T* gamma = reinterpret_cast<const T*>(p.gamma);
+  const T* beta = reinterpret_cast<const T*>(p.beta);
+  uint4 tab[NV], add[NV];
+  auto fetch = [&](long long r, long long id) {
+    const bool ok = id >= 0 && id < p.vocab;                   // an id outside the table reads as a row of zeros and is counted
+    if (!ok && lane == 0 && p.bad) atomicAdd(p.bad, 1);
+    const T* tr = table + (ok ? id : 0) * d;
+    const long long outer = r / p.period;
+    const T* ar = p.add ? reinterpret_cast<const T*>(p.add) + outer * p.s0 + (r - outer * p.period) * p.s1 : nullptr;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (i * 32 + lane) * E;
+      if (c < d) {
+        tab[i] = ok ? __ldg(reinterpret_cast<const uint4*>(tr + c)) : make_uint4(0u, 0u, 0u, 0u);
+        if (ar) add[i] = __ldg(reinterpret_cast<const uint4*>(ar + c));
+      }
+    }
+  };
+  fetch(row, __ldg(p.ids + row));
+  long long idNext = row + step < p.rows ? __ldg(p.ids + row + step) : 0;
+  const float invD = 1.f / (float)d;
+  for (; row < p.rows; row += step) {
+    float v[NV][E];
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (i * 32 + lane) * E;
+      if (c < d) {
+        unpackVec<T, E>(tab[i], v[i]);
+        if (p.add) {
+          float a[E];
+          unpackVec<T, E>(add[i], a);
+#pragma unroll
+          for (int e = 0; e < E; ++e) { v[i][e] += a[e]; if (sizeof(T) == 2) v[i][e] = __bfloat162float(__float2bfloat16_rn(v[i][e])); }
+        }
+#pragma unroll
+        for (int e = 0; e < E; ++e) s += v[i][e];
+      }
+    }
+    if (row + step < p.rows) {
+      fetch(row + step, idNext);
+      if (row + 2 * step < p.rows) idNext = __ldg(p.ids + row + 2 * step);
+    }
+    const float mean = warpSum(s) * invD;
+    float q = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (i * 32 + lane) * E;
+      if (c < d) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) { const float a = v[i][e] - mean; q = fmaf(a, a, q); }
+      }
+    }
+    const float rstd = rsqrtf(warpSum(q) * invD + p.eps);
+    T* orow = reinterpret_cast<T*>(p.out) + row * d;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (i * 32 + lane) * E;
+      if (c < d) {
+        float g[E], b[E], o[E];
+        loadElems<T, E>(gamma + c, g); loadElems<T, E>(beta + c, b);
+#pragma unroll
+        for (int e = 0; e < E; ++e) o[e] = fmaf((v[i][e] - mean) * rstd, g[e], b[e]);
+        storeElems<T, E>(orow + c, o);
+      }
+    }
+  }
+}
+// any row length and alignment: a block per row that reads it three times
+__global__ void __launch_bounds__(256) embed_norm_block_kernel(const __grid_constant__ EmbedNormArgs p, long long d, int dt) {
+  __shared__ float red[32];
+  const long long row = blockIdx.x, id = p.ids[row], outer = row / p.period;
+  const bool ok = id >= 0 && id < p.vocab;
+  if (!ok && threadIdx.x == 0 && p.bad) atomicAdd(p.bad, 1);
+  const long long tBase = (ok ? id : 0) * d, aBase = outer * p.s0 + (row - outer * p.period) * p.s1;
+  auto value = [&](long long c) {
+    float x = ok ? loadAs(p.table, tBase + c, dt) : 0.f;
+    if (p.add) { x += loadAs(p.add, aBase + c, dt); if (dt == LLC_BFLOAT16) x = __bfloat162float(__float2bfloat16_rn(x)); }
+    return x;
+  };
+  auto total = [&](float s) {
+    s = warpSum(s);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    s = 0.f;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
+    return s;
+  };
+  float s = 0.f;
+  for (long long c = threadIdx.x; c < d; c += blockDim.x) s += value(c);
+  const float mean = total(s) / (float)d;
+  float q = 0.f;
+  for (long long c = threadIdx.x; c < d; c += blockDim.x) { const float a = value(c) - mean; q += a * a; }
+  const float rstd = rsqrtf(total(q) / (float)d + p.eps);
+  for (long long c = threadIdx.x; c < d; c += blockDim.x)
+    storeAs(p.out, row * d + c, dt, (value(c) - mean) * rstd * loadAs(p.gamma, c, dt) + loadAs(p.beta, c, dt));
+}
+template <typename T> int launchEmbedNorm(const EmbedNormArgs& a, cudaStream_t st) {
+  constexpr int E = 16 / (int)sizeof(T);
+  const long long wantBlocks = (a.rows + kWarpsPerBlock - 1) / kWarpsPerBlock, cap = (long long)deviceSMs() * 6;
+  const unsigned blocks = (unsigned)(wantBlocks < cap ? wantBlocks : cap);
+  const int nv = (a.d + 32 * E - 1) / (32 * E);
+  if (nv <= 1) embed_norm_kernel<T, 1><<<blocks, kWarpsPerBlock * 32, 0, st>>>(a);
+  else if (nv <= 2) embed_norm_kernel<T, 2><<<blocks, kWarpsPerBlock * 32, 0, st>>>(a);
+  else if (nv <= 3) embed_norm_kernel<T, 3><<<blocks, kWarpsPerBlock * 32, 0, st>>>(a);
+  else if (nv <= 4) embed_norm_kernel<T, 4><<<blocks, kWarpsPerBlock * 32, 0, st>>>(a);
+  else if (nv <= 6) embed_norm_kernel<T, 6><<<blocks, kWarpsPerBlock * 32, 0, st>>>(a);
+  else embed_norm_kernel<T, 8><<<blocks, kWarpsPerBlock * 32, 0, st>>>(a);
+  LLC_LAUNCH_CHECK("embed_norm_kernel");
+  return LLC_OK;
+}
+
 // ---- reductions ------------------------------------------------------------------------------
 __device__ __forceinline__ float redInit(int op) { return op == 1 ? -INFINITY : op == 2 ? INFINITY : 0.f; }
 __device__ __forceinline__ float redOp(float a, float b, int op) { return op == 1 ? fmaxf(a, b) : op == 2 ? fminf(a, b) : a + b; }
@@ -285,6 +417,27 @@ extern "C" int llc_cuda_layernorm(const void* x, const void* gamma, const void* 
   layernorm_block_kernel<<<(unsigned)rows, 256, 0, st>>>(x, gamma, beta, out, idt, pdt, odt, rows, d, eps);
   LLC_LAUNCH_CHECK("layernorm_block_kernel");
   return LLC_OK;
+}
+
+extern "C" int llc_cuda_embed_norm(const LlcEmbedNormParams* p, void* stream) {
+  if (!p) return setError(LLC_ERR_ARGUMENT, "llc argument: embed_norm null parameter block");
+  if (p->rows <= 0 || p->d <= 0) return LLC_OK;
+  if (!p->table || !p->ids || !p->out || !p->gamma || !p->beta) return setError(LLC_ERR_ARGUMENT, "llc argument: embed_norm null pointer");
+  if (p->dtype != LLC_FLOAT32 && p->dtype != LLC_BFLOAT16) return setError(LLC_ERR_UNSUPPORTED, "llc argument: embed_norm type must be f32 or bf16");
+  if (p->add && p->period <= 0) return setError(LLC_ERR_ARGUMENT, "llc argument: embed_norm period must be positive");
+  const int e = p->dtype == LLC_BFLOAT16 ? 8 : 4;
+  const bool fast = p->d % e == 0 && p->d <= 32 * e * 8 && aligned16(p->table) && aligned16(p->out) && aligned16(p->gamma) && aligned16(p->beta) &&
+                    (!p->add || (p->add_s0 % e == 0 && p->add_s1 % e == 0 && aligned16(p->add)));
+  EmbedNormArgs a{};
+  a.table = p->table; a.ids = reinterpret_cast<const long long*>(p->ids); a.add = p->add; a.gamma = p->gamma; a.beta = p->beta; a.out = p->out; a.bad = p->bad_ids;
+  a.rows = p->rows; a.vocab = p->vocab; a.period = p->add ? p->period : p->rows; a.s0 = p->add_s0; a.s1 = p->add_s1; a.d = (int)p->d; a.eps = p->eps;
+  if (!fast) {                                   // caller memory on any boundary, long or odd rows
+    if (p->rows > 2147483647LL) return setError(LLC_ERR_ARGUMENT, "llc argument: embed_norm row count too large");
+    embed_norm_block_kernel<<<(unsigned)p->rows, 256, 0, (cudaStream_t)stream>>>(a, p->d, p->dtype);
+    LLC_LAUNCH_CHECK("embed_norm_block_kernel");
+    return LLC_OK;
+  }
+  return p->dtype == LLC_BFLOAT16 ? launchEmbedNorm<__nv_bfloat16>(a, (cudaStream_t)stream) : launchEmbedNorm<float>(a, (cudaStream_t)stream);
 }
 
 extern "C" int llc_cuda_reduce(const void* x, void* out, int32_t idt, int32_t odt, int64_t outer, int64_t r, int64_t inner, int32_t op, void* stream) {

@@ -1112,12 +1112,14 @@ struct Lowering {
     std::vector<Expr> oshape = it.shape; oshape.push_back(table.shape[1]);
     Expr rows = numelOf(it.shape);
     View idf = ids; idf.shape = {rows}; idf.strides = {Expr(1)};
-    View out = freshView(resultDtype(op->results[0]), oshape, false);
+    // rows of a weight table at constant places (the position embeddings of a fixed length) are looked up once, at load
+    const bool atLoad = bufIsConst(table.buf) && bufIsConst(ids.buf) && numelOf(oshape).isConst();
+    View out = freshView(resultDtype(op->results[0]), oshape, atLoad);
     View o2 = out; o2.shape = {rows, table.shape[1]}; o2.strides = {table.shape[1], Expr(1)};
-    Step s; s.kernel = "gather";
+    Step s; s.kernel = "gather"; s.init = atLoad;
     s.views.emplace_back("table", table); s.views.emplace_back("ids", idf); s.views.emplace_back("out", o2);
     plan.steps.push_back(s);
-    tvs[op->results[0]] = makeView(out, false);
+    tvs[op->results[0]] = makeView(out, atLoad);
   }
   void batchNormInference(Op* op) {
     // y = (x - mean) * gamma / sqrt(var + eps) + beta (src/Dialect/LLH/Transforms/DecomposeOps.cpp:125-144),

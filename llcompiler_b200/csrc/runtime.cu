@@ -107,18 +107,19 @@ struct RView { int buf; long long off; int rank; long long shape[6], strides[6];
 // A plan step resolved for one symbol binding: the kernel's parameter block is filled once, only the
 // pointers (which depend on where the caller's tensors and the arena are) are patched per call.
 struct PtrPatch { void** slot; int buf; long long byteOff; };
-enum StepKind { kGemm, kConv, kPool, kReduce, kSoftmax, kLayerNorm, kGather, kEltwise, kNchw2Nhwc, kAttention };
+enum StepKind { kGemm, kConv, kPool, kReduce, kSoftmax, kLayerNorm, kGather, kEltwise, kNchw2Nhwc, kAttention, kEmbedNorm };
 struct RStep {
   const Step* step;
   std::vector<std::pair<std::string, RView>> views;
   const RView* view(const char* n) const { for (auto& v : views) if (v.first == n) return &v.second; return nullptr; }
   int kind = -1;
-  LlcGemmParams gemm{}; LlcConvParams conv{}; LlcPoolParams pool{}; LlcEltwiseParams elt{}; LlcAttentionParams attn{};
+  LlcGemmParams gemm{}; LlcConvParams conv{}; LlcPoolParams pool{}; LlcEltwiseParams elt{}; LlcAttentionParams attn{}; LlcEmbedNormParams emb{};
   std::string prog;
   void* sp[4] = {nullptr, nullptr, nullptr, nullptr};   // pointer operands of the row kernels
   int sdt[3] = {0, 0, 0}; long long sd[3] = {0, 0, 0}; int sop = 0; float seps = 0.f;
   long long wide[4] = {0, 0, 0, 0};             // nchw2nhwc with a halo: left columns, total columns, h, w
   std::vector<PtrPatch> patches;
+  std::unique_ptr<Step> own;                // a step made at binding time (fused from plan steps); `step` points to it
   RStep() {}
   RStep(const RStep&) = delete;             // patches point into this object
   RStep& operator=(const RStep&) = delete;
@@ -139,6 +140,74 @@ struct Binding {
   int captures = 0;                         // bounded, so that a caller with ever-new addresses stops paying for captures
   ~Binding() { for (auto& g : graphs) if (g.exec) cudaGraphExecDestroy(g.exec); }
 };
+
+// gather -> (add of rows) -> layernorm, where nothing else reads what is between them, becomes one embed_norm step: the kernel
+// holds a row in registers from the lookup to the normalised store (98304 x 768 bf16: three passes of 48, 62 and 56 us).
+// Done when a plan is bound, on concrete extents, so that plans and saved plans stay as they are.
+void fuseEmbeddingNorms(std::vector<std::unique_ptr<RStep>>& steps, const Plan& plan) {
+  auto readers = [&](int buf) {
+    int n = 0;
+    for (auto& s : steps) for (auto& v : s->views) n += v.second.buf == buf && v.first != "out";
+    for (auto& o : plan.outputs) n += o.buf == buf;
+    return n;
+  };
+  auto writer = [&](int buf, size_t before) {                 // the only step that writes `buf`, if there is exactly one
+    int w = -1;
+    for (size_t k = 0; k < steps.size(); ++k) if (const RView* o = steps[k]->view("out")) if (o->buf == buf) w = w == -1 && k < before ? (int)k : -2;
+    return w;
+  };
+  auto denseRows = [](const RView& v, long long rows, long long d) {   // row-major over the whole of a [rows, d] buffer
+    if (v.off != 0 || v.rank < 2 || v.shape[v.rank - 1] != d) return false;
+    long long acc = 1;
+    for (int k = v.rank - 1; k >= 0; --k) { if (v.shape[k] != 1 && v.strides[k] != acc) return false; acc *= v.shape[k]; }
+    return acc == rows * d;
+  };
+  for (size_t i = 0; i < steps.size(); ++i) {
+    const RStep& L = *steps[i];
+    if (L.step->kernel != "layernorm") continue;
+    const RView *xp = L.view("x"), *gp = L.view("gamma"), *bp = L.view("beta"), *op = L.view("out");
+    if (!xp || !gp || !bp || !op || xp->rank != 2) continue;
+    const RView x = *xp, g = *gp, b = *bp, o = *op;
+    if ((x.dtype != LLC_FLOAT32 && x.dtype != LLC_BFLOAT16) || g.dtype != x.dtype || b.dtype != x.dtype || o.dtype != x.dtype) continue;
+    const long long rows = x.shape[0], d = x.shape[1], e = x.dtype == LLC_BFLOAT16 ? 8 : 4;     // elements of a 16-byte vector
+    auto mult = [&](long long v) { return v >= 0 && v % e == 0; };
+    if (rows < 1 || d < 1 || !mult(d) || d > 32 * e * 8 || !mult(g.off) || !mult(b.off) || !mult(o.off) || !denseRows(x, rows, d) || readers(x.buf) != 1) continue;
+    int gi = writer(x.buf, i), ei = -1;
+    if (gi < 0) continue;
+    RView add{}; bool hasAdd = false;
+    if (steps[gi]->step->kernel == "eltwise") {
+      const RStep& E = *steps[gi];
+      const std::string prog = E.step->param("prog");
+      if ((prog != "ld0;ld1;add,0,1" && prog != "ld0;ld1;add,1,0") || E.views.size() != 3 || !denseRows(*E.view("out"), rows, d)) continue;
+      for (int side = 0; side < 2 && !hasAdd; ++side) {
+        const RView t = *E.view(side ? "in1" : "in0");
+        RView a = *E.view(side ? "in0" : "in1");
+        const int w = writer(t.buf, (size_t)gi);
+        if (w < 0 || steps[w]->step->kernel != "gather" || readers(t.buf) != 1 || a.buf == t.buf || t.dtype != x.dtype || a.dtype != x.dtype || !denseRows(t, rows, d)) continue;
+        if (a.rank == 2) { a.rank = 3; a.shape[2] = a.shape[1]; a.shape[1] = a.shape[0]; a.shape[0] = 1; a.strides[2] = a.strides[1]; a.strides[1] = a.strides[0]; a.strides[0] = 0; }
+        if (a.rank != 3 || a.strides[2] != 1 || a.shape[2] != d || a.shape[0] * a.shape[1] != rows || !mult(a.strides[0]) || !mult(a.strides[1]) || !mult(a.off)) continue;
+        add = a; hasAdd = true; ei = gi; gi = w;
+      }
+      if (!hasAdd) continue;
+    }
+    const RStep& G = *steps[gi];
+    if (G.step->kernel != "gather") continue;
+    const RView t = *G.view("table"), ids = *G.view("ids"), go = *G.view("out");
+    if (ids.dtype != LLC_INT64 || t.dtype != x.dtype || go.dtype != x.dtype || t.rank != 2 || t.shape[1] != d || t.strides[1] != 1 || t.strides[0] != d || !mult(t.off) ||
+        !denseRows(go, rows, d)) continue;
+    std::unique_ptr<RStep> f(new RStep());
+    f->own.reset(new Step());
+    f->own->kernel = "embed_norm"; f->own->params = L.step->params;
+    f->step = f->own.get();
+    f->views = {{"table", t}, {"ids", ids}, {"gamma", g}, {"beta", b}, {"out", o}};
+    if (hasAdd) f->views.emplace_back("add", add);
+    steps[i] = std::move(f);
+    const size_t first = (size_t)gi;                           // (the gather comes before the add)
+    if (ei >= 0) steps.erase(steps.begin() + ei);
+    steps.erase(steps.begin() + (long)first);
+    i -= ei >= 0 ? 2 : 1;
+  }
+}
 
 std::vector<int64_t> ints(const std::string& s) {
   std::vector<int64_t> o; std::stringstream ss(s); std::string t;
@@ -310,6 +379,14 @@ void LlcExec::prepare(RStep& rs) {
     if (ids.dtype != LLC_INT64) failArg("gather indices must be int64");
     patch(&rs.sp[0], t); patch(&rs.sp[1], ids); patch(&rs.sp[2], o);
     rs.sdt[0] = t.dtype; rs.sdt[1] = o.dtype; rs.sd[0] = o.shape[0]; rs.sd[1] = o.shape[1]; rs.sd[2] = t.shape[0];
+  } else if (s.kernel == "embed_norm") {
+    rs.kind = kEmbedNorm;
+    const RView &t = need("table"), &ids = need("ids"), &g = need("gamma"), &b = need("beta"), &o = need("out");
+    LlcEmbedNormParams& p = rs.emb;
+    patch(&p.table, t); patch(&p.ids, ids); patch(&p.gamma, g); patch(&p.beta, b); patch(&p.out, o);
+    p.dtype = t.dtype; p.rows = o.shape[0]; p.d = o.shape[1]; p.vocab = t.shape[0]; p.period = 1;
+    if (const RView* a = rs.view("add")) { patch(&p.add, *a); p.period = a->shape[1]; p.add_s0 = a->strides[0]; p.add_s1 = a->strides[1]; }   // [outer, period, d]
+    p.eps = std::stof(s.param("eps", "1e-5")); p.bad_ids = badIds;
   } else if (s.kernel == "nchw2nhwc") {
     rs.kind = kNchw2Nhwc;
     const RView &x = need("x"), &o = need("out");      // both logical [N, C, H, W]
@@ -356,6 +433,7 @@ int LlcExec::launch(RStep& rs, cudaStream_t st) {
     case kSoftmax: return llc_cuda_softmax(rs.sp[0], rs.sp[1], rs.sdt[0], rs.sdt[1], rs.sd[0], rs.sd[1], st);
     case kLayerNorm: return llc_cuda_layernorm(rs.sp[0], rs.sp[1], rs.sp[2], rs.sp[3], rs.sdt[0], rs.sdt[1], rs.sdt[2], rs.sd[0], rs.sd[1], rs.seps, st);
     case kGather: return llc_cuda_gather(rs.sp[0], (const int64_t*)rs.sp[1], rs.sp[2], rs.sdt[0], rs.sdt[1], rs.sd[0], rs.sd[1], rs.sd[2], badIds, st);
+    case kEmbedNorm: return llc_cuda_embed_norm(&rs.emb, st);
     case kEltwise: return llc_cuda_eltwise(&rs.elt, st);
     case kNchw2Nhwc:
       if (rs.wide[1] > 0) return llc_cuda_nchw_to_nhwc_wide(rs.sp[0], rs.sp[1], rs.sdt[0], rs.sd[0], rs.sd[1], rs.wide[2], rs.wide[3], rs.sop, rs.wide[0], rs.wide[1], st);
@@ -434,14 +512,17 @@ Binding& LlcExec::bind(const int64_t* symbols, int nsym, const LlcTensor* in, in
   for (auto& s : plan.steps) {
     if (s.init) continue;
     std::unique_ptr<RStep> rs(new RStep()); rs->step = &s;
-    for (auto& v : s.views) {
-      rs->views.emplace_back(v.first, resolve(v.second, env));
-      int id = v.second.buf, idx = (int)b->steps.size();
-      if (firstUse[id] < 0) firstUse[id] = idx;
-      lastUse[id] = idx;
-    }
-    prepare(*rs);
+    for (auto& v : s.views) rs->views.emplace_back(v.first, resolve(v.second, env));
     b->steps.push_back(std::move(rs));
+  }
+  fuseEmbeddingNorms(b->steps, plan);
+  for (size_t idx = 0; idx < b->steps.size(); ++idx) {
+    for (auto& v : b->steps[idx]->views) {
+      const int id = v.second.buf;
+      if (firstUse[id] < 0) firstUse[id] = (int)idx;
+      lastUse[id] = (int)idx;
+    }
+    prepare(*b->steps[idx]);
   }
   // first-fit packing of temporaries by lifetime
   std::vector<int> temps;

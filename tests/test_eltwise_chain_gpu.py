@@ -63,6 +63,14 @@ def test_rows(dtype, rows, d):
     assert torch.equal(y, (x + a.view(rows, 1, d).float()).abs().to(dtype))
 
 
+def test_rows_of_other_types():
+    m = torch.randint(0, 2, (5, 384), generator=torch.Generator().manual_seed(9)).cuda()
+    for t in (m, m.int(), m.bool(), m.half(), m.to(torch.int8)):
+        out = torch.empty(5, 384, device="cuda")
+        G.eltwise(out, [t], "#1;ld0;cast,1;sub,0,2;#-10000;mul,3,4")
+        assert torch.equal(out, (1.0 - m.float()) * -10000.0)
+
+
 def test_special_values_and_non_chain_programs_agree_with_the_general_path():
     v = torch.tensor([float("nan"), float("inf"), -float("inf"), -0.0, 3.0, -3.0, 1e-40, 65504.0] * 8, device="cuda")
     x, y = v.view(1, 64).repeat(40, 1), v.flip(0).view(64, 1).repeat(1, 40).t()
