@@ -198,9 +198,10 @@ int pairModeEnv() {
 // 0.46 (tf32 0.45 / 0.54), at 0.6 us more for setting up the pair.  98304 x 768 x 3072 bf16 0.372 -> 0.323 ms, 98304 x 2304 x
 // 768 0.264 -> 0.250, 4096 x 768 x 3072 tf32 58 -> 48 us; 6144 x 768 x 768 (one round either way) 19.4 against 21.4 us, which
 // is what the 0.6 is for.  Narrower pair tiles and tf32x3 pairs measured equal to single CTAs and are not built.
-// `wsBytes` > 0 allows split-K: when the tiles of a width leave at least half of the SMs idle and the K loop is long, K
-// is cut into slices that run side by side (every unit resident at once) and meet in the workspace.
-TilePlan chooseTile(long long M, long long N, long long batch, bool allow256, int kind, int kBlocks, long long wsBytes, bool allowPair) {
+// `allowSplit`: K may be cut into up to four slices that run side by side as a cluster and meet in distributed shared memory;
+// meeting costs 3.5 to 9 us by the bytes that cross (24 x 768 x 3072 bf16, 64 columns: 22.5 us whole, 18.4 / 17.1 / 16.4 in
+// two / three / four slices; 128 columns 23.4, 21.1, 19.3, 19.2).
+TilePlan chooseTile(long long M, long long N, long long batch, bool allow256, int kind, int kBlocks, bool allowSplit, bool allowPair) {
   static const float kBlockUs[3][3] = {{0.32f, 0.36f, 0.46f}, {0.33f, 0.37f, 0.54f}, {0.66f, 0.80f, 0.f}};   // [kind][width]
   static const float kPairUs[2] = {0.42f, 0.45f};
   static const float epilogueUs[3] = {0.8f, 1.2f, 2.0f};
@@ -212,19 +213,15 @@ TilePlan chooseTile(long long M, long long N, long long batch, bool allow256, in
     if (bn == 256 && (!allow256 || kind == 2)) continue;
     if (i > 0 && N <= bn / 2) continue;                    // at least half of the tile's columns exist
     const long long tiles = mT * ((N + bn - 1) / bn) * batch;
-    int splits = 1;
-    if (wsBytes > 0 && tiles * 2 <= numSMs() && kBlocks >= 8) {
-      splits = (int)(numSMs() / tiles);
-      if (splits > 4) splits = 4;
-      // a slice keeps at least four K blocks.  With the parked tiles laid out for 512-byte warp accesses, splitting
-      // whenever half of the SMs would idle measured equal or faster on every workload (encoder 128: 0.153 against
-      // 0.162 ms, ResNet-18 1.185 against 1.298 ms without split-K), so there is no minimum slice time any more.
-      while (splits > 1 && (kBlocks / splits < 4 || 4096 + tiles * splits * (long long)BM * bn * 4 > wsBytes)) --splits;
+    for (int splits = 1; splits <= 4; ++splits) {
+      if (splits > 1 && (!allowSplit || kBlocks / splits < 4)) break;      // (four K blocks a slice also mean that none is empty)
+      // every cluster runs at once: pairs fill the chip, wider clusters do not (48 of three took two waves, 34.8 us for 22.5)
+      if (splits > 1 && tiles * splits > (splits == 2 ? numSMs() : numSMs() * 3 / 4)) break;
+      const long long rounds = (tiles * splits + numSMs() - 1) / numSMs();
+      const float loop = ((kBlocks + splits - 1) / splits) * kBlockUs[kind][i];
+      const float cost = (float)rounds * ((loop > epilogueUs[i] ? loop : epilogueUs[i]) + 0.3f) + (splits > 1 ? 2.5f + 0.9f * (float)((splits - 1) << i) + (i > 0 ? 1.5f : 0.f) : 0.f);
+      if (bestCost == 0.f || cost <= bestCost) { best = TilePlan{bn, splits, 1}; bestCost = cost; }
     }
-    const long long rounds = (tiles * splits + numSMs() - 1) / numSMs();
-    const float loop = ((kBlocks + splits - 1) / splits) * kBlockUs[kind][i];
-    const float cost = (float)rounds * ((loop > epilogueUs[i] ? loop : epilogueUs[i]) + 0.3f) + (splits > 1 ? 10.0f : 0.f);
-    if (i == 0 || cost <= bestCost) { best = TilePlan{bn, splits, 1}; bestCost = cost; }
   }
   if (pairMode != 0 && (N > 128 || pairMode == 2)) {
     const long long tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256) * batch, slots = numSMs() / 2;
@@ -272,8 +269,8 @@ int tcGemm(const LlcGemmParams* p, cudaStream_t st) {
   const long long batch = p->b0 * p->b1;
   const bool bmn = p->b_sk != 1;
   const int kind = !f32 ? 0 : (p->precision == LLC_PREC_TF32X3 ? 2 : 1);
-  const bool wsOk = p->workspace && (reinterpret_cast<uintptr_t>(p->workspace) & 15) == 0 && !bmn && splitKEnabled();
-  const TilePlan plan = chooseTile(p->m, p->n, batch, !bmn, kind, (int)((p->k + bk - 1) / bk), wsOk ? p->workspace_bytes : 0, !bmn);
+  const bool allowSplit = p->workspace && !bmn && splitKEnabled();
+  const TilePlan plan = chooseTile(p->m, p->n, batch, !bmn, kind, (int)((p->k + bk - 1) / bk), allowSplit, !bmn);
   const int bn = plan.bn;
   CUtensorMap ma, mb;
   bool okMaps = makeMap(&ma, p->a, f32, p->k, p->m, p->b1, p->b0, p->a_sm, p->a_s1, p->a_s0, BM);
@@ -288,7 +285,7 @@ int tcGemm(const LlcGemmParams* p, cudaStream_t st) {
   a.M = p->m; a.N = p->n; a.K = p->k;
   a.o_s0 = p->o_s0; a.o_s1 = p->o_s1; a.o_sm = p->o_sm; a.r_s0 = p->r_s0; a.r_s1 = p->r_s1; a.r_sm = p->r_sm; a.r_sn = p->r_sn;
   a.b1 = (int)p->b1; a.kBlocks = (int)((p->k + bk - 1) / bk);
-  a.splits = plan.splits; a.counters = reinterpret_cast<int*>(p->workspace); a.ws = reinterpret_cast<float*>(reinterpret_cast<char*>(p->workspace) + 4096);
+  a.splits = plan.splits;
   a.aZ0 = p->b0 > 1 && p->a_s0 > 0; a.aZ1 = p->b1 > 1 && p->a_s1 > 0; a.bZ0 = p->b0 > 1 && p->b_s0 > 0; a.bZ1 = p->b1 > 1 && p->b_s1 > 0;
   const int ob = p->out_dtype == LLC_FLOAT32 ? 4 : 2;
   a.vecOut = (reinterpret_cast<uintptr_t>(p->out) % (ob * 4)) == 0 && p->o_sm % 4 == 0 && p->o_s0 % 4 == 0 && p->o_s1 % 4 == 0;
@@ -333,8 +330,8 @@ int tcConv(const LlcConvParams* p, cudaStream_t st) {
   const int bk = kTileKBytes / eb;
   const long long M = p->n * p->oh * p->ow, K = p->kh * p->kw * p->c;
   const int kind = !f32 ? 0 : (p->precision == LLC_PREC_TF32X3 ? 2 : 1);
-  const bool wsOk = p->workspace && (reinterpret_cast<uintptr_t>(p->workspace) & 15) == 0 && im2colEligible(p, f32) && splitKEnabled();
-  const TilePlan plan = chooseTile(M, p->f, 1, true, kind, (int)((K + bk - 1) / bk), wsOk ? p->workspace_bytes : 0, im2colEligible(p, f32));
+  const bool allowSplit = p->workspace && im2colEligible(p, f32) && splitKEnabled();
+  const TilePlan plan = chooseTile(M, p->f, 1, true, kind, (int)((K + bk - 1) / bk), allowSplit, im2colEligible(p, f32));
   const int bn = plan.bn;
   CUtensorMap mb;
   if (!makeMap(&mb, p->w, f32, K, p->f, 1, 1, K, 0, 0, bn / plan.cg))
@@ -346,7 +343,7 @@ int tcConv(const LlcConvParams* p, cudaStream_t st) {
   a.out_dtype = p->out_dtype; a.res_dtype = p->res_dtype; a.act = p->act; a.alpha = p->alpha;
   a.M = M; a.N = p->f; a.K = K; a.o_sm = p->f; a.r_sm = p->f; a.r_sn = 1; a.b1 = 1;
   a.kBlocks = (int)((K + bk - 1) / bk);
-  a.splits = plan.splits; a.counters = reinterpret_cast<int*>(p->workspace); a.ws = reinterpret_cast<float*>(reinterpret_cast<char*>(p->workspace) + 4096);
+  a.splits = plan.splits;
   const int ob = p->out_dtype == LLC_FLOAT32 ? 4 : 2;
   a.vecOut = (reinterpret_cast<uintptr_t>(p->out) % (ob * 4)) == 0 && p->f % 4 == 0;
   a.x = p->x; a.H = (int)p->h; a.W = (int)p->w_in; a.C = (int)p->c; a.KH = (int)p->kh; a.KW = (int)p->kw; a.OH = (int)p->oh; a.OW = (int)p->ow;

@@ -53,8 +53,7 @@ struct TcArgs {
   long long o_s0, o_s1, o_sm, r_s0, r_s1, r_sm, r_sn;
   int b1; int kBlocks; int vecOut;
   int resTile;              // the residual can be fetched as 32-row x 64-byte units with 16-byte loads
-  int splits;               // K is cut into this many slices, each a work unit of its own; partial tiles meet in `ws`
-  float* ws; int* counters; // split-K: [units][128][BN] partial accumulators; one arrival counter per tile (zero between launches)
+  int splits;               // K is cut into this many slices, each a CTA of one cluster; the partial tiles meet in distributed shared memory
   int hasBLo;               // tf32x3: the low-order part of B comes from memory (mapBLo) instead of the split warps
   int tmaOut;               // 0, or the bytes per row of the output box the epilogue stores through TMA (64)
   int aZ0, aZ1, bZ0, bZ1;   // 1: the operand has this batch dim, 0: it is broadcast (coordinate 0)
@@ -168,7 +167,7 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
   uint64_t* accEmpty = bars + 3 * kStages + 2;  // [2] accumulator drained by the epilogue
   uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 4);
   volatile int* abortWord = reinterpret_cast<volatile int*>(tmemSlot + 1);
-  volatile int* lastFlag = abortWord + 1;       // split-K: whether this CTA's unit arrived last at its tile
+  uint64_t* meet = bars + 31;               // split-K: the other slices' partial tiles are in their CTAs' shared memory
   uint64_t* resFull = bars + 32;                // [8 epilogue warps][4]: a unit of the residual has landed (RES)
   uint8_t* staging = smem + kStages * S::kStageBytes + S::kBarrierBytes;   // 1024-byte aligned
   constexpr int kStagingPerWarp = S::kStagingPerWarp;
@@ -178,18 +177,20 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
   // The CTA (pair)'s share of the work, and the rows of a tile this CTA holds.  In a pair the barriers the issuer waits on
   // (full, accEmpty) are those of CTA 0, the issuer's; what the MMAs signal (empty, accFull) reaches both CTAs.
   const int rank = PAIR ? (int)clusterCtaRank() : 0;
+  const bool clustered = PAIR || p.splits > 1;          // split-K: the grid holds every unit, a cluster the slices of one tile
   const uint32_t unit0 = blockIdx.x / CG, unitStep = gridDim.x / CG;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbarInit(&full[s], kFullCount); mbarInit(&empty[s], 1); mbarInit(&split[s], 4); }
     for (int a = 0; a < 2; ++a) { mbarInit(&accFull[a], 1); mbarInit(&accEmpty[a], kEpiWarps * CG); }
     if (RES) for (int i = 0; i < kEpiWarps * 4; ++i) mbarInit(&resFull[i], 1);
+    else if (p.splits > 1) mbarInit(meet, (uint32_t)(kEpiWarps * (p.splits - 1)));
     *abortWord = 0;
     fenceBarrierInit();
   }
   if (warp == 1) { if constexpr (PAIR) tmemAllocPair(tmemSlot, kAccCols); else tmemAlloc(tmemSlot, kAccCols); }
   tcFenceBefore();
-  if constexpr (PAIR) clusterSync(); else __syncthreads();
+  if (clustered) clusterSync(); else __syncthreads();
   tcFenceAfter();
   const uint32_t tmemBase = *tmemSlot;
 
@@ -455,15 +456,13 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
       tcFenceAfter();
       const uint32_t acc = tmemBase + (uint32_t)(ab * kSetCols) + ((uint32_t)(q * 32) << 16);
       const int usedChains = kb1 - kb0 < kChains ? kb1 - kb0 : kChains;
-      // Split-K: every unit parks its partial tile (fp32, this lane's row) in the workspace; the unit that arrives last
-      // at the tile's counter adds the slices up and runs the epilogue.  Units of one tile run on different CTAs at the
-      // same time (the grid holds every unit), so nobody waits for anybody.
-      const float4* wsRow = nullptr;
-      if (splitK) {
-        // Layout of a parked tile: [epilogue warp][32-column chunk][float4 of the chunk][lane], so that one store (and,
-        // in the unit that adds up, one load) of a warp covers 512 contiguous bytes.  Writer and reader are the same
-        // (warp, lane) position of their CTAs, so the layout needs to make sense to nobody else.
-        float4* mine = reinterpret_cast<float4*>(p.ws + (size_t)u * BM * BN) + (size_t)((half * 4 + q) * (kColsPerWarp / 4)) * 32 + lane;
+      // Split-K: every slice but the first puts its partial tile (fp32) into its own shared memory, where the operand stages
+      // are no longer needed, and is done; the first slice's CTA adds the others to its accumulator in slice order and runs
+      // the epilogue.  Layout: [epilogue warp][32-column chunk][float4 of the chunk][lane], writer and reader being the same
+      // (warp, lane) of their CTAs.  (Through a global workspace with a fence, an arrival counter and the last slice reading
+      // everything back, meeting cost 10 us a tile and overlapping launches raced for it.)
+      float4* const parked = reinterpret_cast<float4*>(tiles) + (size_t)((half * 4 + q) * (kColsPerWarp / 4)) * 32 + lane;
+      if (splitK && clusterCtaRank() != 0) {
 #pragma unroll 1
         for (int ci = 0; ci < kChunks; ++ci) {
           const int c0 = half * kColsPerWarp + ci * 32;
@@ -472,48 +471,32 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
           tmemLoad32x32(acc + (uint32_t)c0, v);
           if (kChains > 1) {
             for (int ch = 1; ch < usedChains; ++ch) {
-              float w[32];
-              tmemLoad32x32(acc + (uint32_t)(ch * BN + c0), w);
+              float w2[32];
+              tmemLoad32x32(acc + (uint32_t)(ch * BN + c0), w2);
 #pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] += w[j];
+              for (int j = 0; j < 32; ++j) v[j] += w2[j];
             }
           }
 #pragma unroll
-          for (int j = 0; j < 8; ++j) __stcg(mine + (ci * 8 + j) * 32, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
+          for (int j = 0; j < 8; ++j) parked[(ci * 8 + j) * 32] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         }
         tcFenceBefore();
         __syncwarp();
-        if (lane == 0) mbarArrive(&accEmpty[ab]);
-        __threadfence();                                 // the partial tile is visible before the arrival is counted
-        asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
-        if (warp == 2 && lane == 0) {
-          int* counter = &p.counters[u / (uint32_t)p.splits];
-          const int old = atomicAdd(counter, 1);
-          const int last = old == p.splits - 1;
-          if (last) *counter = 0;                   // everyone has arrived: the counter is zero again for the next launch
-          *lastFlag = last;
-        }
-        asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
-        if (!*lastFlag) continue;
-        __threadfence();
-        wsRow = reinterpret_cast<const float4*>(p.ws + (size_t)(u / (uint32_t)p.splits * (uint32_t)p.splits) * BM * BN) + (size_t)((half * 4 + q) * (kColsPerWarp / 4)) * 32 + lane;
-        if (resTile) issueRes(0);
+        if (lane == 0) { mbarArrive(&accEmpty[ab]); mbarArriveLeaderRelease(meet); }
+        continue;                                          // (a CTA has one unit)
       }
-      const bool pipelined = kPrefetch && !splitK;
+      if (splitK) {
+        if (resTile) issueRes(0);
+        if (!mbarWaitCluster(meet, 0, abortWord)) atomicExch(p.status, 4);
+      }
+      const bool pipelined = kPrefetch;
       uint32_t raw[32];
       if (pipelined) { __syncwarp(); tmemIssue32(acc + (uint32_t)(half * kColsPerWarp), raw); }
 #pragma unroll 1
       for (int ci = 0; ci < kChunks; ++ci) {
         const int c0 = half * kColsPerWarp + ci * 32;
         float v[32];
-        if (splitK) {                                   // the slices' partial sums, from the workspace (L2)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) { const float4 f = __ldcg(wsRow + (ci * 8 + j) * 32); v[4 * j] = f.x; v[4 * j + 1] = f.y; v[4 * j + 2] = f.z; v[4 * j + 3] = f.w; }
-          for (int sl = 1; sl < p.splits; ++sl) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) { const float4 f = __ldcg(wsRow + (size_t)sl * (BM * BN / 4) + (ci * 8 + j) * 32); v[4 * j] += f.x; v[4 * j + 1] += f.y; v[4 * j + 2] += f.z; v[4 * j + 3] += f.w; }
-          }
-        } else if (pipelined) {
+        if (pipelined) {
           tmemWait32(raw);
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
@@ -530,7 +513,13 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
             }
           }
         }
-        if (!splitK && ci == kChunks - 1) {             // this warp's share is in registers: hand the accumulator back
+        if (splitK) {                                   // the other slices' partial sums
+          for (int sl = 1; sl < p.splits; ++sl) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) { const float4 f = loadPeer4(parked + (ci * 8 + j) * 32, (uint32_t)sl); v[4 * j] += f.x; v[4 * j + 1] += f.y; v[4 * j + 2] += f.z; v[4 * j + 3] += f.w; }
+          }
+        }
+        if (ci == kChunks - 1) {                        // this warp's share is in registers: hand the accumulator back
           tcFenceBefore();
           __syncwarp();
           if (lane == 0) { if constexpr (PAIR) mbarArriveLeader(&accEmpty[ab]); else mbarArrive(&accEmpty[ab]); }
@@ -782,8 +771,9 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
   }
   tcFenceBefore();
   __syncwarp();
-  // (pair: neither CTA leaves while the other's MMAs may read its shared memory or arrive on its barriers)
-  if constexpr (PAIR) clusterSync(); else __syncthreads();
+  // (neither CTA of a pair leaves while the other's MMAs may read its shared memory or arrive on its barriers, and no slice
+  // before its partial tile has been read)
+  if (clustered) clusterSync(); else __syncthreads();
   if (warp == 1) { tcFenceAfter(); if constexpr (PAIR) tmemDeallocPair(tmemBase, kAccCols); else tmemDealloc(tmemBase, kAccCols); }
 }
 
@@ -823,9 +813,10 @@ int launchTc(const TcMaps& m, TcArgs a, long long batch, cudaStream_t st) {
   cfg.dynamicSmemBytes = S::kTotal;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
-  if (CG == 2) {
+  const int cluster = CG == 2 ? 2 : a.splits;
+  if (cluster > 1) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
   }
   LLC_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, m.a, m.b, m.out, m.bLo, m.res, a));
