@@ -39,8 +39,9 @@ typedef struct LlcGemmParams {
   int64_t r_s0, r_s1, r_sm, r_sn;
   float alpha;
   int32_t act;         /* LlcAct */
-  /* NULL disables split-K on the tensor cores (few output tiles, long K).  The memory itself is not touched any more: the
-   * slices of a tile meet in shared memory, so launches may overlap whatever is given here. */
+  /* Optional scratch for K slices (few output tiles, long K): device memory, 16-byte
+   * aligned, whose first 4096 bytes are zero before the first use (the kernel leaves them zero).
+   * NULL disables them.  Launches that share one workspace must not overlap on the GPU. */
   void* workspace;
   int64_t workspace_bytes;
   /* Optional, precision tf32x3 only: B - truncate_to_tf32(B), laid out exactly like b (same strides).  When given, the
@@ -101,7 +102,8 @@ typedef struct LlcConvParams {
    * which turns a filter row of a narrow-channel convolution into the channels of a 1-wide kernel.  Tensor-core precisions
    * only (bf16, tf32, tf32x3); c * element size must then be a multiple of 16 bytes and so must the strides. */
   int64_t x_sn, x_sh, x_sw;
-  /* NULL disables split-K (few output tiles, long K), as in LlcGemmParams; the memory itself is not touched. */
+  /* Optional scratch for K slices (few output tiles, long K), as in LlcGemmParams: device memory, 16-byte aligned, first
+   * 4096 bytes zero before the first use (left zero).  NULL disables them. */
   void* workspace;
   int64_t workspace_bytes;
 } LlcConvParams;

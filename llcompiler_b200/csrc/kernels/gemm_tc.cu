@@ -191,6 +191,45 @@ int pairModeEnv() {
   return e && *e ? atoi(e) : 1;
 }
 
+// LLC_TC_SLICES=n cuts K into n slices wherever they can run (the tests use it to reach every way of meeting).
+int slicesEnv() {
+  const char* e = getenv("LLC_TC_SLICES");
+  return e && *e ? atoi(e) : 0;
+}
+
+int ceilDiv(long long a, long long b) { return (int)((a + b - 1) / b); }
+// Accumulators a unit always has: tf32x3 spreads its K blocks over 256 columns of tensor memory.
+int setAccs(int kind, int bn) { return kind == 2 ? 256 / bn : 1; }
+
+// Workspace of a call cut into K slices: 4096 bytes of arrival counters and the parked partial tiles.
+long long parkedBytes(long long tiles, int splits, int bn) { return 4096 + tiles * splits * (long long)BM * bn * 4; }
+
+// K blocks one accumulator may sum up.  The tensor core truncates what it adds, so the error of a result grows with the
+// length of its sums (64 x 128 x 1024 bf16 against float64: 1.0e-6 of the result as one sum, 2.3e-7 as four), and a plan
+// that is chosen by time alone would trade accuracy for it.  The line: a call whose tiles leave at least half of the SMs idle
+// sums what up to four K slices over the idle SMs would, of at least four K blocks, at the width that is fastest when
+// slices meet in memory at 10 us a tile.  chooseTile reaches it by slices or by accumulators.
+int longestChain(long long M, long long N, long long batch, bool allow256, int kind, int kBlocks, long long wsBytes) {
+  static const float kBlockUs[3][3] = {{0.22f, 0.25f, 0.40f}, {0.28f, 0.33f, 0.50f}, {0.60f, 0.75f, 0.f}};   // [kind][width]
+  static const float epilogueUs[3] = {0.8f, 1.2f, 2.0f};
+  int chain = kBlocks; float bestCost = 0.f;
+  for (int i = 0; i < 3; ++i) {
+    const int bn = 64 << i;
+    if (bn == 256 && (!allow256 || kind == 2)) continue;
+    if (i > 0 && N <= bn / 2) continue;
+    const long long tiles = (M + BM - 1) / BM * ((N + bn - 1) / bn) * batch;
+    int splits = 1;
+    if (wsBytes > 0 && tiles * 2 <= numSMs() && kBlocks >= 8) {
+      splits = (int)(numSMs() / tiles < 4 ? numSMs() / tiles : 4);
+      while (splits > 1 && (kBlocks / splits < 4 || parkedBytes(tiles, splits, bn) > wsBytes)) --splits;
+    }
+    const float loop = ceilDiv(kBlocks, splits) * kBlockUs[kind][i];
+    const float cost = (float)((tiles * splits + numSMs() - 1) / numSMs()) * ((loop > epilogueUs[i] ? loop : epilogueUs[i]) + 0.3f) + (splits > 1 ? 10.f : 0.f);
+    if (i == 0 || cost <= bestCost) { chain = ceilDiv(ceilDiv(kBlocks, splits), setAccs(kind, bn)); bestCost = cost; }
+  }
+  return chain;
+}
+
 // Tile by a cost model: a persistent CTA (pair) works through ceil(tiles / slots) tiles, and a tile costs the longer of its
 // main loop (K blocks x a per-block time that grows slowly with the width, because narrow tiles are bound by operand
 // traffic and latency rather than by the tensor pipe) and its epilogue.  Times in microseconds, measured on B200.
@@ -198,38 +237,52 @@ int pairModeEnv() {
 // 0.46 (tf32 0.45 / 0.54), at 0.6 us more for setting up the pair.  98304 x 768 x 3072 bf16 0.372 -> 0.323 ms, 98304 x 2304 x
 // 768 0.264 -> 0.250, 4096 x 768 x 3072 tf32 58 -> 48 us; 6144 x 768 x 768 (one round either way) 19.4 against 21.4 us, which
 // is what the 0.6 is for.  Narrower pair tiles and tf32x3 pairs measured equal to single CTAs and are not built.
-// `allowSplit`: K may be cut into up to four slices that run side by side as a cluster and meet in distributed shared memory;
-// meeting costs 3.5 to 9 us by the bytes that cross (24 x 768 x 3072 bf16, 64 columns: 22.5 us whole, 18.4 / 17.1 / 16.4 in
-// two / three / four slices; 128 columns 23.4, 21.1, 19.3, 19.2).
-TilePlan chooseTile(long long M, long long N, long long batch, bool allow256, int kind, int kBlocks, bool allowSplit, bool allowPair) {
+// `wsBytes` > 0 allows slices: where the tiles leave SMs idle, K may be cut into up to four that run side by side, one unit
+// per CTA, and meet in the workspace, 3.5 to 10.5 us by the bytes that are parked.  (As clusters that met in distributed
+// shared memory 1024 x 768 x 3072 tf32x3 had only two slices and took 44.5 us; in three, through memory, 34.7.)
+TilePlan chooseTile(long long M, long long N, long long batch, bool allow256, int kind, int kBlocks, long long wsBytes, bool allowPair) {
   static const float kBlockUs[3][3] = {{0.32f, 0.36f, 0.46f}, {0.33f, 0.37f, 0.54f}, {0.66f, 0.80f, 0.f}};   // [kind][width]
   static const float kPairUs[2] = {0.42f, 0.45f};
   static const float epilogueUs[3] = {0.8f, 1.2f, 2.0f};
-  const int pairMode = kind == 2 || !allowPair || !allow256 ? 0 : pairModeEnv();
+  const int pairMode = kind == 2 || !allowPair || !allow256 ? 0 : pairModeEnv(), forced = wsBytes > 0 ? slicesEnv() : 0;
+  const int chain = longestChain(M, N, batch, allow256, kind, kBlocks, wsBytes);
   const long long mT = (M + BM - 1) / BM;
-  TilePlan best{64, 1, 1}; float bestCost = 0.f;
+  TilePlan best{64, 1, 1, setAccs(kind, 64), false}; float bestCost = 0.f;
   for (int i = 0; i < 3; ++i) {
     const int bn = 64 << i;
     if (bn == 256 && (!allow256 || kind == 2)) continue;
     if (i > 0 && N <= bn / 2) continue;                    // at least half of the tile's columns exist
     const long long tiles = mT * ((N + bn - 1) / bn) * batch;
     for (int splits = 1; splits <= 4; ++splits) {
-      if (splits > 1 && (!allowSplit || kBlocks / splits < 4)) break;      // (four K blocks a slice also mean that none is empty)
-      // every cluster runs at once: pairs fill the chip, wider clusters do not (48 of three took two waves, 34.8 us for 22.5)
-      if (splits > 1 && tiles * splits > (splits == 2 ? numSMs() : numSMs() * 3 / 4)) break;
+      if (splits > 1 && (kBlocks / splits < 4 || tiles * splits > numSMs())) break;      // (four K blocks a slice also mean that none is empty)
+      if (splits > 1 && parkedBytes(tiles, splits, bn) > wsBytes) break;
+      if (forced && splits != forced) continue;
+      const int perSlice = ceilDiv(kBlocks, splits), set = setAccs(kind, bn);
+      const int accs = ceilDiv(perSlice, chain) > set ? ceilDiv(perSlice, chain) : set;
+      if (accs > set && (wsBytes <= 0 || tiles * splits > numSMs() || accs * bn > 512)) continue;        // accumulators beyond the set's: one unit per CTA
       const long long rounds = (tiles * splits + numSMs() - 1) / numSMs();
-      const float loop = ((kBlocks + splits - 1) / splits) * kBlockUs[kind][i];
-      const float cost = (float)rounds * ((loop > epilogueUs[i] ? loop : epilogueUs[i]) + 0.3f) + (splits > 1 ? 2.5f + 0.9f * (float)((splits - 1) << i) + (i > 0 ? 1.5f : 0.f) : 0.f);
-      if (bestCost == 0.f || cost <= bestCost) { best = TilePlan{bn, splits, 1}; bestCost = cost; }
+      const float loop = perSlice * kBlockUs[kind][i];
+      const float cost = (float)rounds * ((loop > epilogueUs[i] ? loop : epilogueUs[i]) + 0.3f) + (splits > 1 ? 2.5f + 0.5f * (float)(splits << i) : 0.f);
+      if (bestCost == 0.f || cost <= bestCost) { best = TilePlan{bn, splits, 1, accs, splits > 1 || accs > set}; bestCost = cost; }
     }
   }
-  if (pairMode != 0 && (N > 128 || pairMode == 2)) {
+  if (pairMode != 0 && !forced && (N > 128 || pairMode == 2)) {
     const long long tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256) * batch, slots = numSMs() / 2;
     const float loop = kBlocks * kPairUs[kind];
     const float cost = (float)((tiles + slots - 1) / slots) * ((loop > epilogueUs[2] ? loop : epilogueUs[2]) + 0.3f) + 0.6f;
-    if (cost <= bestCost || pairMode == 2) best = TilePlan{256, 1, 2};
+    if (pairMode == 2 || (chain >= kBlocks && cost <= bestCost)) best = TilePlan{256, 1, 2, 1, false};
   }
   return best;
+}
+
+// The plan as the kernel reads it.
+void setPlan(TcArgs& a, const TilePlan& plan, void* workspace) {
+  a.splits = plan.splits; a.accs = plan.accs; a.accBlocks = ceilDiv(ceilDiv(a.kBlocks, plan.splits), plan.accs);
+  if (plan.splits > 1) { a.counters = reinterpret_cast<int*>(workspace); a.ws = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + 4096); }
+}
+// Bytes of a caller's workspace that slices can meet in.
+long long usableWorkspace(const void* workspace, long long bytes) {
+  return workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && splitKEnabled() ? bytes : 0;
 }
 
 }  // namespace
@@ -269,8 +322,7 @@ int tcGemm(const LlcGemmParams* p, cudaStream_t st) {
   const long long batch = p->b0 * p->b1;
   const bool bmn = p->b_sk != 1;
   const int kind = !f32 ? 0 : (p->precision == LLC_PREC_TF32X3 ? 2 : 1);
-  const bool allowSplit = p->workspace && !bmn && splitKEnabled();
-  const TilePlan plan = chooseTile(p->m, p->n, batch, !bmn, kind, (int)((p->k + bk - 1) / bk), allowSplit, !bmn);
+  const TilePlan plan = chooseTile(p->m, p->n, batch, !bmn, kind, (int)((p->k + bk - 1) / bk), bmn ? 0 : usableWorkspace(p->workspace, p->workspace_bytes), !bmn);
   const int bn = plan.bn;
   CUtensorMap ma, mb;
   bool okMaps = makeMap(&ma, p->a, f32, p->k, p->m, p->b1, p->b0, p->a_sm, p->a_s1, p->a_s0, BM);
@@ -285,7 +337,7 @@ int tcGemm(const LlcGemmParams* p, cudaStream_t st) {
   a.M = p->m; a.N = p->n; a.K = p->k;
   a.o_s0 = p->o_s0; a.o_s1 = p->o_s1; a.o_sm = p->o_sm; a.r_s0 = p->r_s0; a.r_s1 = p->r_s1; a.r_sm = p->r_sm; a.r_sn = p->r_sn;
   a.b1 = (int)p->b1; a.kBlocks = (int)((p->k + bk - 1) / bk);
-  a.splits = plan.splits;
+  setPlan(a, plan, p->workspace);
   a.aZ0 = p->b0 > 1 && p->a_s0 > 0; a.aZ1 = p->b1 > 1 && p->a_s1 > 0; a.bZ0 = p->b0 > 1 && p->b_s0 > 0; a.bZ1 = p->b1 > 1 && p->b_s1 > 0;
   const int ob = p->out_dtype == LLC_FLOAT32 ? 4 : 2;
   a.vecOut = (reinterpret_cast<uintptr_t>(p->out) % (ob * 4)) == 0 && p->o_sm % 4 == 0 && p->o_s0 % 4 == 0 && p->o_s1 % 4 == 0;
@@ -301,7 +353,7 @@ int tcGemm(const LlcGemmParams* p, cudaStream_t st) {
   // the residual through a ring of TMA loads: whole tiles only (no split-K), same element type as the output
   CUtensorMap mr = mo;
   bool resRing = false;
-  if (a.resTile && a.tmaOut && plan.splits == 1 && kind != 2 && !bmn && resRingEnabled()) {
+  if (a.resTile && a.tmaOut && !plan.cut && kind != 2 && !bmn && resRingEnabled()) {
     bool h1 = false, h0 = false;
     if (makeResMap(&mr, p->res, ob == 4, p->n, p->m, p->b1, p->b0, p->r_sm, p->r_s1, p->r_s0, &h1, &h0)) { resRing = true; a.rZ1 = h1; a.rZ0 = h0; }
   }
@@ -330,8 +382,7 @@ int tcConv(const LlcConvParams* p, cudaStream_t st) {
   const int bk = kTileKBytes / eb;
   const long long M = p->n * p->oh * p->ow, K = p->kh * p->kw * p->c;
   const int kind = !f32 ? 0 : (p->precision == LLC_PREC_TF32X3 ? 2 : 1);
-  const bool allowSplit = p->workspace && im2colEligible(p, f32) && splitKEnabled();
-  const TilePlan plan = chooseTile(M, p->f, 1, true, kind, (int)((K + bk - 1) / bk), allowSplit, im2colEligible(p, f32));
+  const TilePlan plan = chooseTile(M, p->f, 1, true, kind, (int)((K + bk - 1) / bk), im2colEligible(p, f32) ? usableWorkspace(p->workspace, p->workspace_bytes) : 0, im2colEligible(p, f32));
   const int bn = plan.bn;
   CUtensorMap mb;
   if (!makeMap(&mb, p->w, f32, K, p->f, 1, 1, K, 0, 0, bn / plan.cg))
@@ -343,7 +394,7 @@ int tcConv(const LlcConvParams* p, cudaStream_t st) {
   a.out_dtype = p->out_dtype; a.res_dtype = p->res_dtype; a.act = p->act; a.alpha = p->alpha;
   a.M = M; a.N = p->f; a.K = K; a.o_sm = p->f; a.r_sm = p->f; a.r_sn = 1; a.b1 = 1;
   a.kBlocks = (int)((K + bk - 1) / bk);
-  a.splits = plan.splits;
+  setPlan(a, plan, p->workspace);
   const int ob = p->out_dtype == LLC_FLOAT32 ? 4 : 2;
   a.vecOut = (reinterpret_cast<uintptr_t>(p->out) % (ob * 4)) == 0 && p->f % 4 == 0;
   a.x = p->x; a.H = (int)p->h; a.W = (int)p->w_in; a.C = (int)p->c; a.KH = (int)p->kh; a.KW = (int)p->kw; a.OH = (int)p->oh; a.OW = (int)p->ow;
@@ -362,7 +413,7 @@ int tcConv(const LlcConvParams* p, cudaStream_t st) {
     if (makeIm2colMap(&ma, p, f32)) {
       CUtensorMap mr = mo;
       bool resRing = false;
-      if (a.resTile && a.tmaOut && plan.splits == 1 && kind != 2 && resRingEnabled()) {
+      if (a.resTile && a.tmaOut && !plan.cut && kind != 2 && resRingEnabled()) {
         bool h1 = false, h0 = false;
         if (makeResMap(&mr, p->res, ob == 4, p->f, M, 1, 1, p->f, 0, 0, &h1, &h0)) resRing = true;
       }
@@ -370,8 +421,7 @@ int tcConv(const LlcConvParams* p, cudaStream_t st) {
       return kind == 0 ? dispatchTc<2, 0>(plan, resRing, maps, a, 1, st) : kind == 1 ? dispatchTc<2, 1>(plan, resRing, maps, a, 1, st) : dispatchTc<2, 2>(plan, false, maps, a, 1, st);
     }
   }
-  a.splits = 1;                                          // the gathered form walks whole tiles
-  if (plan.cg != 1) return setError(LLC_ERR_CUDA, "llc cuda: cuTensorMapEncodeIm2col rejected the convolution input");
+  if (plan.cg != 1 || plan.cut) return setError(LLC_ERR_CUDA, "llc cuda: cuTensorMapEncodeIm2col rejected the convolution input");
   const TcMaps maps{mb, mb, mo, mbl, mo};
   return kind == 0 ? dispatchTc<1, 0>(plan, false, maps, a, 1, st) : kind == 1 ? dispatchTc<1, 1>(plan, false, maps, a, 1, st) : dispatchTc<1, 2>(plan, false, maps, a, 1, st);
 }

@@ -53,7 +53,9 @@ struct TcArgs {
   long long o_s0, o_s1, o_sm, r_s0, r_s1, r_sm, r_sn;
   int b1; int kBlocks; int vecOut;
   int resTile;              // the residual can be fetched as 32-row x 64-byte units with 16-byte loads
-  int splits;               // K is cut into this many slices, each a CTA of one cluster; the partial tiles meet in distributed shared memory
+  int splits;               // K is cut into this many slices, each a CTA of its own; partial tiles meet in `ws`
+  float* ws; int* counters; // workspace: parked partial tiles, and one arrival counter per tile (zero between launches)
+  int accs, accBlocks;      // accumulators a unit's K loop is spread over, added up in the epilogue; bf16 / tf32: each sums this many K blocks in a row
   int hasBLo;               // tf32x3: the low-order part of B comes from memory (mapBLo) instead of the split warps
   int tmaOut;               // 0, or the bytes per row of the output box the epilogue stores through TMA (64)
   int aZ0, aZ1, bZ0, bZ1;   // 1: the operand has this batch dim, 0: it is broadcast (coordinate 0)
@@ -127,7 +129,10 @@ __host__ __device__ constexpr int tcThreads(int kind, int mode) { return (2 + kE
 // bytes lies inside one filter tap: channels * element size is a multiple of 128).  (A variant with sixteen epilogue
 // warps and one pipeline stage less was measured 1.2 to 1.9 times slower on every shape tried and is not kept.)
 // CG: 1, a CTA works for itself on 128 x BN tiles; 2, a cluster of two CTAs works on 256 x BN tiles with cta_group::2 MMAs.
-template <int BN, int KIND, int MODE, bool BMN, bool RES, int CG>
+// CUT: calls of few tiles, one unit per CTA: K cut into slices that meet in the workspace, or sums spread over more accumulators
+// than the set has, or both.  A variant of its own, because the code for it in the others' epilogue cost them 2 % (bottleneck
+// block, 256 images 451 -> 459 us).
+template <int BN, int KIND, int MODE, bool BMN, bool RES, int CG, bool CUT>
 __global__ void __launch_bounds__(tcThreads(KIND, MODE), 1)
 tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapO,
           const __grid_constant__ CUtensorMap mapBLo, const __grid_constant__ CUtensorMap mapR, const TcArgs p) {
@@ -138,18 +143,22 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
   constexpr bool PAIR = CG == 2;
   using S = Smem<BN, KIND, RES, CG>;
   static_assert(!PAIR || (MODE != 1 && !BMN && KIND != 2), "CTA pairs take TMA-fed K-major bf16 / tf32 operands");
+  static_assert(!CUT || (MODE != 1 && !BMN && !RES && !PAIR), "one-CTA tiles of TMA-fed K-major operands can be cut along K");
   static_assert(!RES || (KIND != 2 && MODE != 1 && !BMN), "the residual ring exists for bf16 / tf32 kernels with TMA-fed operands");
   constexpr int kStages = S::kStages;
   constexpr int kElemBytes = TF32 ? 4 : 2;
   constexpr int BK = kTileKBytes / kElemBytes;          // 64 bf16 / 32 tf32
   constexpr int UMMA_K = 32 / kElemBytes;               // 16 bf16 / 8 tf32 (32 bytes of K per instruction)
   constexpr uint32_t kIdesc = instrDesc(TF32 ? 2 : 1, CG * BM, BN, 0, BMN ? 1 : 0);
-  // Two accumulator sets (double buffering).  tf32x3 splits the K loop over kChains independent
-  // accumulators per set and adds them in the epilogue: the tensor core truncates when it adds into
-  // its fp32 accumulator, so shorter chains mean a smaller (K-proportional) rounding bias.
+  // Two accumulator sets (double buffering).  The tensor core truncates when it adds into its fp32 accumulator, so shorter
+  // chains mean a smaller (K-proportional) rounding bias: tf32x3 spreads the K loop over kChains accumulators per set and
+  // adds them in the epilogue; the CUT kernels spread it over p.accs of them (chooseTile says how many), past the first set,
+  // which nothing else uses where a CTA has one unit.
   constexpr int kChains = X3 ? 256 / BN : 1;
   constexpr int kSetCols = X3 ? 256 : BN;
-  constexpr int kAccCols = 2 * kSetCols;
+  const int accs = CUT ? p.accs : kChains;
+  uint32_t accCols = 2 * kSetCols;                             // tensor memory to hold (twice as much cost 0.2 us a launch)
+  if (CUT) while ((int)accCols < accs * BN) accCols *= 2;
   static_assert(!X3 || BN <= 128, "tf32x3 uses BN <= 128");
   constexpr int kAtomN = kTileKBytes / kElemBytes;      // BMN: elements of n per 128-byte slab row
   constexpr int kSlabBytes = BK * 128;                  // BMN: one slab = BK rows of k x 128 bytes of n
@@ -167,7 +176,7 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
   uint64_t* accEmpty = bars + 3 * kStages + 2;  // [2] accumulator drained by the epilogue
   uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 4);
   volatile int* abortWord = reinterpret_cast<volatile int*>(tmemSlot + 1);
-  uint64_t* meet = bars + 31;               // split-K: the other slices' partial tiles are in their CTAs' shared memory
+  volatile int* lastFlag = reinterpret_cast<volatile int*>(tmemSlot + 2);   // split-K: this CTA's slice arrived last
   uint64_t* resFull = bars + 32;                // [8 epilogue warps][4]: a unit of the residual has landed (RES)
   uint8_t* staging = smem + kStages * S::kStageBytes + S::kBarrierBytes;   // 1024-byte aligned
   constexpr int kStagingPerWarp = S::kStagingPerWarp;
@@ -177,20 +186,18 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
   // The CTA (pair)'s share of the work, and the rows of a tile this CTA holds.  In a pair the barriers the issuer waits on
   // (full, accEmpty) are those of CTA 0, the issuer's; what the MMAs signal (empty, accFull) reaches both CTAs.
   const int rank = PAIR ? (int)clusterCtaRank() : 0;
-  const bool clustered = PAIR || p.splits > 1;          // split-K: the grid holds every unit, a cluster the slices of one tile
   const uint32_t unit0 = blockIdx.x / CG, unitStep = gridDim.x / CG;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbarInit(&full[s], kFullCount); mbarInit(&empty[s], 1); mbarInit(&split[s], 4); }
     for (int a = 0; a < 2; ++a) { mbarInit(&accFull[a], 1); mbarInit(&accEmpty[a], kEpiWarps * CG); }
     if (RES) for (int i = 0; i < kEpiWarps * 4; ++i) mbarInit(&resFull[i], 1);
-    else if (p.splits > 1) mbarInit(meet, (uint32_t)(kEpiWarps * (p.splits - 1)));
     *abortWord = 0;
     fenceBarrierInit();
   }
-  if (warp == 1) { if constexpr (PAIR) tmemAllocPair(tmemSlot, kAccCols); else tmemAlloc(tmemSlot, kAccCols); }
+  if (warp == 1) { if constexpr (PAIR) tmemAllocPair(tmemSlot, accCols); else tmemAlloc(tmemSlot, accCols); }
   tcFenceBefore();
-  if (clustered) clusterSync(); else __syncthreads();
+  if (PAIR) clusterSync(); else __syncthreads();
   tcFenceAfter();
   const uint32_t tmemBase = *tmemSlot;
 
@@ -272,13 +279,19 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
         if (!waitIssuer(&accEmpty[ab], aph ^ 1)) { atomicExch(p.status, 2); ok = false; break; }
         tcFenceAfter();
         const uint32_t accSet = tmemBase + (uint32_t)(ab * kSetCols);
+        uint32_t cutAcc = accSet; int inChain = 0;          // CUT: where this K block's accumulator lies (divisions here held the MMAs up, 17 -> 20 us for 300 x 256 x 4096 tf32)
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % kStages; const uint32_t ph = (it / kStages) & 1;
           if (!waitIssuer(X3 ? &split[s] : &full[s], ph)) { atomicExch(p.status, 2); ok = false; break; }
           if (CONV && !X3) fenceProxyAsync();               // the gathered A tile was written through the generic proxy
           tcFenceAfter();
-          const uint32_t acc = accSet + (uint32_t)(((kb - kb0) % kChains) * BN);
-          const bool fresh = kb - kb0 < kChains;           // first K block of this chain: overwrite
+          const uint32_t acc = CUT ? cutAcc : accSet + (uint32_t)(((kb - kb0) % kChains) * BN);
+          const bool fresh = X3 || !CUT ? kb - kb0 < accs : inChain == 0;      // first K block of this chain: overwrite
+          if constexpr (CUT) {                              // tf32x3 takes the accumulators in turn, the other kinds one after the other
+            ++inChain;
+            if (X3) { cutAcc += BN; if (inChain == accs) { inChain = 0; cutAcc = accSet; } }
+            else if (inChain == p.accBlocks) { inChain = 0; cutAcc += BN; }
+          }
           const uint64_t dA = smemDescKMajorSw128(smemAddr(stageA(s)));
           const uint64_t dB = BMN ? smemDescMnMajorSw128(smemAddr(stageB(s)), kSlabBytes) : smemDescKMajorSw128(smemAddr(stageB(s)));
           constexpr uint64_t kAdvA = (UMMA_K * kElemBytes) >> 4;                      // 32 bytes of K inside the swizzle atom
@@ -316,7 +329,7 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
     const int q = warp & 3, half = (warp - 2) >> 2;
     constexpr int kColsPerWarp = BN / (kEpiWarps / 4);
     constexpr int kChunks = kColsPerWarp / 32;
-    constexpr bool kPrefetch = kChains == 1 && !CONV;           // tf32x3 adds several accumulators per chunk, and the gather form has no registers to spare
+    constexpr bool kPrefetch = kChains == 1 && !CONV && !CUT;   // tf32x3 and CUT add several sums per chunk, and the gather form has no registers to spare
     constexpr uint32_t kRing = (uint32_t)S::kSlots;
     char* outBase = reinterpret_cast<char*>(p.out);
     const bool outF32 = p.out_dtype == LLC_FLOAT32;
@@ -360,7 +373,7 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
     uint32_t tcount = 0;
     for (uint32_t u = unit0; u < units; u += unitStep, ++tcount) {
       int kb0, kb1; kRange(w, kb0, kb1);
-      const int tileM = w.m, tileN = w.n, zb0 = w.z0, zb1 = w.z1;
+      const int tileM = w.m, tileN = w.n, zb0 = w.z0, zb1 = w.z1, sliceIdx = w.s;
       w.next(p);
       if (affine) {
         asm volatile("bar.sync %0, 128;" ::"r"(3 + half) : "memory");      // the previous tile's factors have been read
@@ -450,76 +463,81 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
                        "r"(*reinterpret_cast<const unsigned*>(&a3)) : "memory");
         }
       };
-      const bool splitK = !RES && !PAIR && p.splits > 1;
+      const bool splitK = CUT && p.splits > 1;
       if (resTile && !splitK) issueRes(0);
       if (!mbarWait(&accFull[ab], aph, abortWord)) atomicExch(p.status, 4);   // carry on with whatever is there: every warp must still reach the barriers below
       tcFenceAfter();
       const uint32_t acc = tmemBase + (uint32_t)(ab * kSetCols) + ((uint32_t)(q * 32) << 16);
-      const int usedChains = kb1 - kb0 < kChains ? kb1 - kb0 : kChains;
-      // Split-K: every slice but the first puts its partial tile (fp32) into its own shared memory, where the operand stages
-      // are no longer needed, and is done; the first slice's CTA adds the others to its accumulator in slice order and runs
-      // the epilogue.  Layout: [epilogue warp][32-column chunk][float4 of the chunk][lane], writer and reader being the same
-      // (warp, lane) of their CTAs.  (Through a global workspace with a fence, an arrival counter and the last slice reading
-      // everything back, meeting cost 10 us a tile and overlapping launches raced for it.)
-      float4* const parked = reinterpret_cast<float4*>(tiles) + (size_t)((half * 4 + q) * (kColsPerWarp / 4)) * 32 + lane;
-      if (splitK && clusterCtaRank() != 0) {
+      const int usedAccs = X3 ? (kb1 - kb0 < accs ? kb1 - kb0 : accs) : CUT ? (kb1 - kb0 + p.accBlocks - 1) / p.accBlocks : 1;
+      auto loadAccs = [&](int c0, float* v) {           // the unit's sums, 32 columns from c0 on (the load is warp-collective)
+        __syncwarp();
+        tmemLoad32x32(acc + (uint32_t)c0, v);
+        if (X3 || CUT) {
+#pragma unroll 1
+          for (int a = 1; a < usedAccs; ++a) {
+            float w2[32];
+            tmemLoad32x32(acc + (uint32_t)(a * BN + c0), w2);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] += w2[j];
+          }
+        }
+      };
+      // Split-K: every slice parks its partial tile (fp32, this lane's row) in the workspace; the one that arrives last at
+      // the tile's counter adds the slices up in order and runs the epilogue.  The slices of a tile run on different CTAs at
+      // the same time (the grid holds every unit), so nobody waits for anybody.  Layout of a parked tile: [epilogue warp]
+      // [32-column chunk][float4 of the chunk][lane], writer and reader being the same (warp, lane) of their CTAs, so that
+      // one store or load of a warp covers 512 contiguous bytes.  (Clusters that meet in distributed shared memory instead
+      // measured the same, 128 x 768 x 3072 bf16 11.1 against 11.4 us, and 48 clusters of three do not run at once.)
+      const float4* const slices = reinterpret_cast<const float4*>(p.ws) + (size_t)(u - (uint32_t)sliceIdx) * (BM * BN / 4) +
+                                   (size_t)((half * 4 + q) * (kColsPerWarp / 4)) * 32 + lane;        // slice 0 of this tile
+      if (splitK) {
+        float4* const mine = const_cast<float4*>(slices) + (size_t)sliceIdx * (BM * BN / 4);
 #pragma unroll 1
         for (int ci = 0; ci < kChunks; ++ci) {
           const int c0 = half * kColsPerWarp + ci * 32;
           float v[32];
-          __syncwarp();
-          tmemLoad32x32(acc + (uint32_t)c0, v);
-          if (kChains > 1) {
-            for (int ch = 1; ch < usedChains; ++ch) {
-              float w2[32];
-              tmemLoad32x32(acc + (uint32_t)(ch * BN + c0), w2);
+          loadAccs(c0, v);
 #pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] += w2[j];
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j) parked[(ci * 8 + j) * 32] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          for (int j = 0; j < 8; ++j) __stcg(mine + (ci * 8 + j) * 32, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
         }
         tcFenceBefore();
         __syncwarp();
-        if (lane == 0) { mbarArrive(&accEmpty[ab]); mbarArriveLeaderRelease(meet); }
-        continue;                                          // (a CTA has one unit)
-      }
-      if (splitK) {
+        if (lane == 0) mbarArrive(&accEmpty[ab]);
+        __threadfence();                                   // the partial tile is visible before the arrival is counted
+        asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
+        if (warp == 2 && lane == 0) {
+          const int tile = (int)(u / (uint32_t)p.splits), before = atomicAdd(&p.counters[tile], 1);
+          if (before == p.splits - 1) p.counters[tile] = 0;   // everyone has arrived: zero again for the next launch
+          *lastFlag = before == p.splits - 1;
+        }
+        asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
+        if (!*lastFlag) continue;
+        __threadfence();
         if (resTile) issueRes(0);
-        if (!mbarWaitCluster(meet, 0, abortWord)) atomicExch(p.status, 4);
       }
-      const bool pipelined = kPrefetch;
+      constexpr bool pipelined = kPrefetch;
       uint32_t raw[32];
       if (pipelined) { __syncwarp(); tmemIssue32(acc + (uint32_t)(half * kColsPerWarp), raw); }
 #pragma unroll 1
       for (int ci = 0; ci < kChunks; ++ci) {
         const int c0 = half * kColsPerWarp + ci * 32;
         float v[32];
-        if (pipelined) {
+        if (splitK) {                                   // every slice's partial sums, this CTA's own among them (from L2)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) { const float4 f = __ldcg(slices + (ci * 8 + j) * 32); v[4 * j] = f.x; v[4 * j + 1] = f.y; v[4 * j + 2] = f.z; v[4 * j + 3] = f.w; }
+          for (int sl = 1; sl < p.splits; ++sl) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) { const float4 f = __ldcg(slices + (size_t)sl * (BM * BN / 4) + (ci * 8 + j) * 32); v[4 * j] += f.x; v[4 * j + 1] += f.y; v[4 * j + 2] += f.z; v[4 * j + 3] += f.w; }
+          }
+        } else if (pipelined) {
           tmemWait32(raw);
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
           if (ci + 1 < kChunks) { __syncwarp(); tmemIssue32(acc + (uint32_t)(c0 + 32), raw); }
         } else {
-          __syncwarp();                                 // the load is warp-collective
-          tmemLoad32x32(acc + (uint32_t)c0, v);
-          if (kChains > 1) {
-            for (int ch = 1; ch < usedChains; ++ch) {
-              float w[32];
-              tmemLoad32x32(acc + (uint32_t)(ch * BN + c0), w);
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] += w[j];
-            }
-          }
+          loadAccs(c0, v);
         }
-        if (splitK) {                                   // the other slices' partial sums
-          for (int sl = 1; sl < p.splits; ++sl) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) { const float4 f = loadPeer4(parked + (ci * 8 + j) * 32, (uint32_t)sl); v[4 * j] += f.x; v[4 * j + 1] += f.y; v[4 * j + 2] += f.z; v[4 * j + 3] += f.w; }
-          }
-        }
-        if (ci == kChunks - 1) {                        // this warp's share is in registers: hand the accumulator back
+        if (ci == kChunks - 1 && !splitK) {             // this warp's share is in registers: hand the accumulator back
           tcFenceBefore();
           __syncwarp();
           if (lane == 0) { if constexpr (PAIR) mbarArriveLeader(&accEmpty[ab]); else mbarArrive(&accEmpty[ab]); }
@@ -771,14 +789,13 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
   }
   tcFenceBefore();
   __syncwarp();
-  // (neither CTA of a pair leaves while the other's MMAs may read its shared memory or arrive on its barriers, and no slice
-  // before its partial tile has been read)
-  if (clustered) clusterSync(); else __syncthreads();
-  if (warp == 1) { tcFenceAfter(); if constexpr (PAIR) tmemDeallocPair(tmemBase, kAccCols); else tmemDealloc(tmemBase, kAccCols); }
+  // (neither CTA of a pair leaves while the other's MMAs may read its shared memory or arrive on its barriers)
+  if (PAIR) clusterSync(); else __syncthreads();
+  if (warp == 1) { tcFenceAfter(); if constexpr (PAIR) tmemDeallocPair(tmemBase, accCols); else tmemDealloc(tmemBase, accCols); }
 }
 
-// The tile a call is cut into: width, K slices, CTAs per tile.
-struct TilePlan { int bn; int splits; int cg; };
+// The tile a call is cut into: width, K slices, CTAs per tile, accumulators per unit, and whether the CUT kernels take it.
+struct TilePlan { int bn; int splits; int cg; int accs; bool cut; };
 struct TcMaps { CUtensorMap a, b, out, bLo, res; };
 
 // Launches the kernel for one MODE and KIND (see tc_kernel); each pair is compiled in a file of its own.  `res`: the variant
@@ -791,13 +808,13 @@ LLC_TC_DECLARE(2, 0) LLC_TC_DECLARE(2, 1) LLC_TC_DECLARE(2, 2)
 int dispatchTcMn(const TilePlan& plan, const TcMaps& m, const TcArgs& a, long long batch, cudaStream_t st);
 
 // One instantiation: set up once per device, then launched.  CG == 2: clusters of two CTAs, one pair per two SMs.
-template <int BN, int KIND, int MODE, bool BMN, bool RES, int CG>
+template <int BN, int KIND, int MODE, bool BMN, bool RES, int CG, bool CUT>
 int launchTc(const TcMaps& m, TcArgs a, long long batch, cudaStream_t st) {
   using S = Smem<BN, KIND, RES, CG>;
   static_assert(S::kStages >= 2, "at least two pipeline stages");
   static DeviceOnce configured;                          // the shared-memory opt-in is kept per device
   const int dev = currentDevice();
-  auto kernel = tc_kernel<BN, KIND, MODE, BMN, RES, CG>;
+  auto kernel = tc_kernel<BN, KIND, MODE, BMN, RES, CG, CUT>;
   if (!configured.test(dev)) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal);
     if (e != cudaSuccess) return cudaFail(e, "cudaFuncSetAttribute(tc_kernel)");
@@ -805,25 +822,26 @@ int launchTc(const TcMaps& m, TcArgs a, long long batch, cudaStream_t st) {
   }
   a.mTiles = (int)((a.M + CG * BM - 1) / (CG * BM)); a.nTiles = (int)((a.N + BN - 1) / BN);
   a.tiles = (long long)a.mTiles * a.nTiles * batch;
-  if (a.splits < 1 || RES || CG == 2) a.splits = 1;
+  if (!CUT) a.splits = 1;
   const long long units = a.tiles * a.splits, slots = deviceSMs() / CG;
+  if (CUT && (units > slots || a.accs < 1 || a.accs * BN > 512)) return setError(LLC_ERR_INTERNAL, "llc internal: a call cut along K has one unit per CTA");
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)((units < slots ? units : slots) * CG));
   cfg.blockDim = dim3(tcThreads(KIND, MODE));
   cfg.dynamicSmemBytes = S::kTotal;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
-  const int cluster = CG == 2 ? 2 : a.splits;
-  if (cluster > 1) {
+  if (CG == 2) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
   }
   LLC_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, m.a, m.b, m.out, m.bLo, m.res, a));
   return LLC_OK;
 }
 
-#define LLC_TC_CASE(BN_, R_, CG_) if (plan.bn == BN_ && res == R_ && plan.cg == CG_) return launchTc<BN_, KIND, MODE, false, R_, CG_>(m, a, batch, st);
+#define LLC_TC_CASE(BN_, R_, CG_) if (plan.bn == BN_ && res == R_ && plan.cg == CG_ && !plan.cut) return launchTc<BN_, KIND, MODE, false, R_, CG_, false>(m, a, batch, st);
+#define LLC_TC_CUT(BN_) if (plan.bn == BN_ && plan.cut) return launchTc<BN_, KIND, MODE, false, false, 1, true>(m, a, batch, st);
 #define LLC_TC_DISPATCH(MODE_, KIND_, CASES)                                                                                                             \
   template <> int dispatchTc<MODE_, KIND_>(const TilePlan& plan, bool res, const TcMaps& m, const TcArgs& a, long long batch, cudaStream_t st) {          \
     constexpr int MODE = MODE_, KIND = KIND_;                                                                                                            \

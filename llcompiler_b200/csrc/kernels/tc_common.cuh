@@ -82,22 +82,6 @@ __device__ __forceinline__ void mbarArriveLeader(uint64_t* bar) {
       "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}"
       ::"r"(smemAddr(bar)) : "memory");
 }
-// The same with what this warp's threads wrote before (ordered by a __syncwarp) visible to the thread that waits for it.
-__device__ __forceinline__ void mbarArriveLeaderRelease(uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .b32 a;\n\t"
-      "fence.acq_rel.cluster;\n\t"
-      "mapa.shared::cluster.u32 a, %0, 0;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [a];\n\t}"
-      ::"r"(smemAddr(bar)) : "memory");
-}
-// Sixteen bytes at the same place of another CTA of the cluster.
-__device__ __forceinline__ float4 loadPeer4(const void* p, uint32_t rank) {
-  float4 v; uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smemAddr(p)), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
-}
 // The shared::cluster address of the same place in the even CTA of the pair: bit 24 of a CTA's shared addresses is its rank's parity.
 __device__ __forceinline__ uint32_t leaderAddr(const void* p) { return smemAddr(p) & 0xFEFFFFFFu; }
 // Tiled / im2col loads into this CTA's shared memory whose bytes are counted by the barrier of CTA 0 of the pair.

@@ -233,8 +233,8 @@ struct LlcExec {
   int* hostStatus = nullptr;                  // page-locked mirror: [tensor-core word, attention word, bad embedding ids, blockwise attention word]
   bool usesTc = false, usesGather = false;    // which of the words this plan's kernels can write
   std::mutex mutex;                           // one call at a time per executor (bindings, arena and staging are shared state)
-  char* workspace = nullptr;                  // split-K scratch (counters at the head stay zero between launches)
-  static constexpr size_t kWorkspaceBytes = 16u << 20;
+  char* workspace = nullptr;                  // scratch for K slices (counters at the head stay zero between launches): 4096 bytes + a 128 x 256 fp32 tile per SM
+  static constexpr size_t kWorkspaceBytes = 20u << 20;
   cudaStream_t capStream = nullptr;         // capture happens here, so that the legacy default stream can replay too
   std::map<std::vector<int64_t>, std::unique_ptr<Binding>> bindings;
   int64_t lastLaunches = 0;
