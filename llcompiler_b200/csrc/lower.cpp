@@ -505,11 +505,12 @@ struct Lowering {
   // A lazy tree that repeats itself along some dims (every leaf is broadcast there) is computed once per distinct element
   // and read back through stride 0.  An attention mask [b,1,1,n] added to [b,h,m,n] scores is the case that matters: at its
   // full extent it was written out by a step of its own (1.8 GB for 256 x 12 x 384 x 384) and sent the attention kernel
-  // to its per-row mask form, 7.7 ms of a 9.1 ms encoder layer.  False: the tree has no such dim.
-  bool compactBroadcast(const TV& t, View& out) {
+  // to its per-row mask form, 7.7 ms of a 9.1 ms encoder layer.  `keepLast`: the last dim stays at its extent.  False: the
+  // tree has no such dim.
+  bool compactBroadcast(const TV& t, bool keepLast, View& out) {
     if (t.kind != TV::Lazy || nodes[t.root].kind != ENode::Op || treeIsConst(t.root)) return false;
     std::vector<bool> repeats(t.shape.size());
-    for (size_t d = 0; d < t.shape.size(); ++d) repeats[d] = !t.shape[d].isConst(1);
+    for (size_t d = 0; d < t.shape.size(); ++d) repeats[d] = !t.shape[d].isConst(1) && !(keepLast && d + 1 == t.shape.size());
     bool fits = true;
     std::function<void(int)> scan = [&](int id) {
       const ENode& n = nodes[id];
@@ -588,8 +589,10 @@ struct Lowering {
       if (ot.kind == TV::Pending && ot.pending == pt.pending) return false;
       View ov2;
       if (isLeafOnly(ot)) ov2 = nodes[ot.root].leaf;
+      // (only where a broadcast residual is taken below; fused attention reads its mask along the keys, and scores that lose
+      // it are stored in bf16, where a large offset on a whole row leaves nothing of them)
       else if (P.step.kernel == "gemm" && ov->users.size() == 1 && pt.view.shape == P.nativeOut.shape && pt.view.strides == P.nativeOut.strides &&
-               ot.shape == pt.shape && compactBroadcast(ot, ov2)) {}      // (only where a broadcast residual is taken below)
+               ot.shape == pt.shape && compactBroadcast(ot, attentionScores(pt), ov2)) {}
       else { toView(ot); ov2 = ot.view; }
       std::vector<int64_t> cast; size_t off = pt.shape.size() - ot.shape.size();
       for (size_t i = 0; i < ot.shape.size(); ++i) cast.push_back((int64_t)(off + i));

@@ -20,7 +20,7 @@ class _Scores(torch.nn.Module):
 @pytest.mark.parametrize("mask_shape,elements", [((2, 1, 1, 24), 48), ((2, 1, 16, 24), 768), ((1, 3, 1, 1), 3), ((1, 1, 16, 1), 16), ((2, 3, 16, 24), 2304), ((1, 1, 1, 1), 1)])
 def test_masks_of_every_broadcast_form(dtype, mask_shape, elements):
     if dtype is torch.bfloat16 and mask_shape[3] == 1:
-        pytest.skip("an offset of -100 on whole rows is below bf16's resolution of the scores")
+        elements *= 24                                   # fused attention reads masks along the keys: there they keep their extent
     g = torch.Generator().manual_seed(3)
     q, k, v = (torch.randn(2, n, 3, 64, generator=g).to(dtype) for n in (16, 24, 24))
     m = torch.randint(0, 2, mask_shape, generator=g)
@@ -31,8 +31,32 @@ def test_masks_of_every_broadcast_form(dtype, mask_shape, elements):
     assert max_rel_err(got, want) < (1e-5 if dtype is torch.float32 else 2e-2)
     steps = [s for s in comp.compiled[0].engine.text.splitlines() if s.startswith("step eltwise") and "#-100" in s]
     assert len(steps) == 1
+    # bf16 attention is one step, with fp32 scores, for every form of mask (offsets on whole rows of bf16 scores lose them)
+    assert ("step attention" in comp.compiled[0].engine.text) == (dtype is torch.bfloat16)
     out = steps[0].split("out=")[1].split("[")[1].split(";")[0]
     assert math.prod(int(e) for e in out.split(",")) == elements, steps[0]
+
+
+@pytest.mark.parametrize("offset", [-1.0, -100.0, -10000.0])
+@pytest.mark.parametrize("mask_shape", [(2, 1, 16, 1), (1, 3, 1, 1), (16, 1), (1, 1, 1, 1), (2, 1, 1, 24), (24,)])
+def test_masks_do_not_cost_bf16_attention_its_fp32_scores(mask_shape, offset):
+    """An offset that is the same for all keys of a row changes nothing: the error stays that of bf16 operands and results
+    (2^-8 of the largest value), however large the offset is."""
+    class Scores(torch.nn.Module):
+        def forward(self, q, k, v, m):
+            q, k, v = (t.permute(0, 2, 1, 3) for t in (q, k, v))
+            s = torch.matmul(q, k.transpose(-1, -2)) / math.sqrt(64) + (1.0 - m.to(q.dtype)) * offset
+            return torch.matmul(torch.softmax(s, dim=-1), v)
+
+    g = torch.Generator().manual_seed(3)
+    q, k, v = (torch.randn(2, n, 3, 64, generator=g).bfloat16() for n in (16, 24, 24))
+    m = torch.randint(0, 2, mask_shape, generator=g)
+    comp = InterpreterCompiler()
+    fn = compile_with(comp, Scores(), False)
+    with torch.no_grad():
+        got, want = fn(q, k, v, m), Scores()(q.double(), k.double(), v.double(), m)
+    assert max_rel_err(got, want) < 2 * 2.0 ** -8        # (probabilities and results are rounded to bf16)
+    assert "step attention" in comp.compiled[0].engine.text
 
 
 class _Residual(torch.nn.Module):
