@@ -382,9 +382,11 @@ int tcConv(const LlcConvParams* p, cudaStream_t st) {
   const int bk = kTileKBytes / eb;
   const long long M = p->n * p->oh * p->ow, K = p->kh * p->kw * p->c;
   const int kind = !f32 ? 0 : (p->precision == LLC_PREC_TF32X3 ? 2 : 1);
-  const TilePlan plan = chooseTile(M, p->f, 1, true, kind, (int)((K + bk - 1) / bk), im2colEligible(p, f32) ? usableWorkspace(p->workspace, p->workspace_bytes) : 0, im2colEligible(p, f32));
+  // the plan comes after the map: a refused one leaves the gathered form, whose tiles are not cut and not paired
+  CUtensorMap ma, mb;
+  const bool im2col = im2colEligible(p, f32) && makeIm2colMap(&ma, p, f32);
+  const TilePlan plan = chooseTile(M, p->f, 1, true, kind, (int)((K + bk - 1) / bk), im2col ? usableWorkspace(p->workspace, p->workspace_bytes) : 0, im2col);
   const int bn = plan.bn;
-  CUtensorMap mb;
   if (!makeMap(&mb, p->w, f32, K, p->f, 1, 1, K, 0, 0, bn / plan.cg))
     return setError(LLC_ERR_CUDA, "llc cuda: cuTensorMapEncodeTiled rejected the convolution weights");
   TcArgs a{};
@@ -408,20 +410,16 @@ int tcConv(const LlcConvParams* p, cudaStream_t st) {
   a.resTile = p->res && p->res_dtype == p->out_dtype && (reinterpret_cast<uintptr_t>(p->res) & 15) == 0 && (p->f * ob) % 16 == 0;
   CUtensorMap mbl = mb;
   if (kind == 2 && p->w_lo && (reinterpret_cast<uintptr_t>(p->w_lo) & 15) == 0 && makeMap(&mbl, p->w_lo, f32, K, p->f, 1, 1, K, 0, 0, bn / plan.cg)) a.hasBLo = 1;
-  if (im2colEligible(p, f32)) {
-    CUtensorMap ma;
-    if (makeIm2colMap(&ma, p, f32)) {
-      CUtensorMap mr = mo;
-      bool resRing = false;
-      if (a.resTile && a.tmaOut && !plan.cut && kind != 2 && resRingEnabled()) {
-        bool h1 = false, h0 = false;
-        if (makeResMap(&mr, p->res, ob == 4, p->f, M, 1, 1, p->f, 0, 0, &h1, &h0)) resRing = true;
-      }
-      const TcMaps maps{ma, mb, mo, mbl, mr};
-      return kind == 0 ? dispatchTc<2, 0>(plan, resRing, maps, a, 1, st) : kind == 1 ? dispatchTc<2, 1>(plan, resRing, maps, a, 1, st) : dispatchTc<2, 2>(plan, false, maps, a, 1, st);
+  if (im2col) {
+    CUtensorMap mr = mo;
+    bool resRing = false;
+    if (a.resTile && a.tmaOut && !plan.cut && kind != 2 && resRingEnabled()) {
+      bool h1 = false, h0 = false;
+      if (makeResMap(&mr, p->res, ob == 4, p->f, M, 1, 1, p->f, 0, 0, &h1, &h0)) resRing = true;
     }
+    const TcMaps maps{ma, mb, mo, mbl, mr};
+    return kind == 0 ? dispatchTc<2, 0>(plan, resRing, maps, a, 1, st) : kind == 1 ? dispatchTc<2, 1>(plan, resRing, maps, a, 1, st) : dispatchTc<2, 2>(plan, false, maps, a, 1, st);
   }
-  if (plan.cg != 1 || plan.cut) return setError(LLC_ERR_CUDA, "llc cuda: cuTensorMapEncodeIm2col rejected the convolution input");
   const TcMaps maps{mb, mb, mo, mbl, mo};
   return kind == 0 ? dispatchTc<1, 0>(plan, false, maps, a, 1, st) : kind == 1 ? dispatchTc<1, 1>(plan, false, maps, a, 1, st) : dispatchTc<1, 2>(plan, false, maps, a, 1, st);
 }
