@@ -82,8 +82,12 @@ __device__ __forceinline__ void mbarArriveLeader(uint64_t* bar) {
       "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}"
       ::"r"(smemAddr(bar)) : "memory");
 }
-// The shared::cluster address of the same place in the even CTA of the pair: bit 24 of a CTA's shared addresses is its rank's parity.
-__device__ __forceinline__ uint32_t leaderAddr(const void* p) { return smemAddr(p) & 0xFEFFFFFFu; }
+// The shared::cluster address of the same place in CTA 0 of the pair.
+__device__ __forceinline__ uint32_t leaderAddr(const void* p) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smemAddr(p)));
+  return a;
+}
 // Tiled / im2col loads into this CTA's shared memory whose bytes are counted by the barrier of CTA 0 of the pair.
 __device__ __forceinline__ void tmaLoadPair4d(void* smemDst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
   asm volatile(
