@@ -238,12 +238,13 @@ int longestChain(long long M, long long N, long long batch, bool allow256, int k
 // 768 0.264 -> 0.250, 4096 x 768 x 3072 tf32 58 -> 48 us; 6144 x 768 x 768 (one round either way) 19.4 against 21.4 us, which
 // is what the 0.6 is for.  Narrower pair tiles and tf32x3 pairs measured equal to single CTAs and are not built.
 // `wsBytes` > 0 allows slices: where the tiles leave SMs idle, K may be cut into up to four that run side by side, one unit
-// per CTA, and meet in the workspace, 3.5 to 10.5 us by the bytes that are parked.  (As clusters that met in distributed
+// per CTA, and meet in the workspace, 3.5 to 13 us by the bytes that are parked.  (As clusters that met in distributed
 // shared memory 1024 x 768 x 3072 tf32x3 had only two slices and took 44.5 us; in three, through memory, 34.7.)
 TilePlan chooseTile(long long M, long long N, long long batch, bool allow256, int kind, int kBlocks, long long wsBytes, bool allowPair) {
   static const float kBlockUs[3][3] = {{0.32f, 0.36f, 0.46f}, {0.33f, 0.37f, 0.54f}, {0.66f, 0.80f, 0.f}};   // [kind][width]
   static const float kPairUs[2] = {0.42f, 0.45f};
   static const float epilogueUs[3] = {0.8f, 1.2f, 2.0f};
+  static const float meetingUs[3] = {2.5f, 2.5f, 3.f}, parkUs[3] = {0.5f, 1.f, 2.6f};
   const int pairMode = kind == 2 || !allowPair || !allow256 ? 0 : pairModeEnv(), forced = wsBytes > 0 ? slicesEnv() : 0;
   const int chain = longestChain(M, N, batch, allow256, kind, kBlocks, wsBytes);
   const long long mT = (M + BM - 1) / BM;
@@ -262,7 +263,7 @@ TilePlan chooseTile(long long M, long long N, long long batch, bool allow256, in
       if (accs > set && (wsBytes <= 0 || tiles * splits > numSMs() || accs * bn > 512)) continue;        // accumulators beyond the set's: one unit per CTA
       const long long rounds = (tiles * splits + numSMs() - 1) / numSMs();
       const float loop = perSlice * kBlockUs[kind][i];
-      const float cost = (float)rounds * ((loop > epilogueUs[i] ? loop : epilogueUs[i]) + 0.3f) + (splits > 1 ? 2.5f + 0.5f * (float)(splits << i) : 0.f);
+      const float cost = (float)rounds * ((loop > epilogueUs[i] ? loop : epilogueUs[i]) + 0.3f) + (splits > 1 ? meetingUs[i] + parkUs[i] * (float)splits : 0.f);
       if (bestCost == 0.f || cost <= bestCost) { best = TilePlan{bn, splits, 1, accs, splits > 1 || accs > set}; bestCost = cost; }
     }
   }

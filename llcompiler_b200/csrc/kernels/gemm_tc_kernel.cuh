@@ -473,8 +473,20 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
         __syncwarp();
         tmemLoad32x32(acc + (uint32_t)c0, v);
         if (X3 || CUT) {
+          int a = 1;
+          if constexpr (!X3) {                          // two loads in flight
 #pragma unroll 1
-          for (int a = 1; a < usedAccs; ++a) {
+            for (; a + 1 < usedAccs; a += 2) {
+              uint32_t w2[32], w3[32];
+              tmemIssue32(acc + (uint32_t)(a * BN + c0), w2);
+              tmemIssue32(acc + (uint32_t)((a + 1) * BN + c0), w3);
+              tmemWait32(w2); tmemWait32(w3);
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = v[j] + __uint_as_float(w2[j]) + __uint_as_float(w3[j]);
+            }
+          }
+#pragma unroll 1
+          for (; a < usedAccs; ++a) {
             float w2[32];
             tmemLoad32x32(acc + (uint32_t)(a * BN + c0), w2);
 #pragma unroll
@@ -500,6 +512,7 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
 #pragma unroll
           for (int j = 0; j < 8; ++j) __stcg(mine + (ci * 8 + j) * 32, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
         }
+        if (resTile) issueRes(0);                          // (lands under the meeting; the slices that come first need none of it)
         tcFenceBefore();
         __syncwarp();
         if (lane == 0) mbarArrive(&accEmpty[ab]);
@@ -513,7 +526,6 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
         asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * 32) : "memory");
         if (!*lastFlag) continue;
         __threadfence();
-        if (resTile) issueRes(0);
       }
       constexpr bool pipelined = kPrefetch;
       uint32_t raw[32];
@@ -522,12 +534,29 @@ tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
       for (int ci = 0; ci < kChunks; ++ci) {
         const int c0 = half * kColsPerWarp + ci * 32;
         float v[32];
-        if (splitK) {                                   // every slice's partial sums, this CTA's own among them (from L2)
+        if (splitK) {                                   // the partial sums of all two to four slices in order (from L2), two slices in flight
+          float4 even[8], odd[8];
+          auto fetch = [&](int sl, float4* f) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) { const float4 f = __ldcg(slices + (ci * 8 + j) * 32); v[4 * j] = f.x; v[4 * j + 1] = f.y; v[4 * j + 2] = f.z; v[4 * j + 3] = f.w; }
-          for (int sl = 1; sl < p.splits; ++sl) {
+            for (int j = 0; j < 8; ++j) f[j] = __ldcg(slices + (size_t)sl * (BM * BN / 4) + (ci * 8 + j) * 32);
+          };
+          auto add = [&](const float4* f) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) { const float4 f = __ldcg(slices + (size_t)sl * (BM * BN / 4) + (ci * 8 + j) * 32); v[4 * j] += f.x; v[4 * j + 1] += f.y; v[4 * j + 2] += f.z; v[4 * j + 3] += f.w; }
+            for (int j = 0; j < 8; ++j) { v[4 * j] += f[j].x; v[4 * j + 1] += f[j].y; v[4 * j + 2] += f[j].z; v[4 * j + 3] += f[j].w; }
+          };
+          fetch(0, even);
+          if (!X3) fetch(1, odd);                       // (the split warps leave tf32x3 no registers for it)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) { v[4 * j] = even[j].x; v[4 * j + 1] = even[j].y; v[4 * j + 2] = even[j].z; v[4 * j + 3] = even[j].w; }
+          if constexpr (X3) {
+#pragma unroll 1
+            for (int sl = 1; sl < p.splits; ++sl) { fetch(sl, odd); add(odd); }
+          } else {
+            if (p.splits > 2) fetch(2, even);
+            add(odd);
+            if (p.splits > 3) fetch(3, odd);
+            if (p.splits > 2) add(even);
+            if (p.splits > 3) add(odd);
           }
         } else if (pipelined) {
           tmemWait32(raw);
