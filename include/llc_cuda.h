@@ -52,9 +52,13 @@ int llc_cuda_gemm(const LlcGemmParams* p, void* stream);
 
 /* llc_cuda_gemm on the FMA path for callers that must not allocate device memory (a process whose
  * own pool already owns the GPU, a loop that cannot take the synchronisation an allocation
- * implies).  No counterpart in the reference.  `workspace` in the parameter block is ignored.  A shape
- * whose K slices would take more than 1 MiB of partial tiles is refused with LLC_ERR_ARGUMENT.  Calls
- * share nothing and may overlap.  Calls no cudaMalloc / cudaFree. */
+ * implies).  No counterpart in the reference.  The split-K scratch is a 1 MiB array built into the
+ * library (each GPU that loads the library holds it until exit); `workspace` in the parameter block
+ * is ignored.  A shape whose split needs more than 1 MiB is refused with LLC_ERR_ARGUMENT.  The
+ * first call on a device looks up the array's device address (cudaGetSymbolAddress); make that
+ * first call before starting any stream capture.  All calls share the one array: launches that
+ * overlap on the GPU (different streams or threads of one process on one device) race.
+ * Calls no cudaMalloc / cudaFree. */
 int llc_cuda_gemm_static_scratch(const LlcGemmParams* p, void* stream);
 
 /* out[b0,b1,m,:] = softmax_n(scale * sum_d Q[b0,b1,m,d] K[b0,b1,n,d] + mask[b0,b1,m,n]) V[b0,b1,n,:] in one kernel: the

@@ -3,7 +3,7 @@
 #include "common.cuh"
 
 namespace llc {
-int simtGemm(const LlcGemmParams* p, cudaStream_t st);
+int igemmSimtGemm(const LlcGemmParams* p, cudaStream_t st, void* workspace, long long workspaceBytes);
 int igemmSimtConv(const LlcConvParams* p, cudaStream_t st);
 bool tcGemmSupported(const LlcGemmParams* p);
 int tcGemm(const LlcGemmParams* p, cudaStream_t st);
@@ -25,7 +25,7 @@ extern "C" int llc_cuda_gemm(const LlcGemmParams* p, void* stream) {
   if (!floatIo(p->in_dtype) || !floatIo(p->out_dtype) || (p->res && !floatIo(p->res_dtype)))
     return setError(LLC_ERR_UNSUPPORTED, "llc argument: gemm operands must be f32 or bf16");
   if (tcGemmSupported(p)) return tcGemm(p, (cudaStream_t)stream);
-  return simtGemm(p, (cudaStream_t)stream);
+  return igemmSimtGemm(p, (cudaStream_t)stream, p->workspace, p->workspace_bytes);
 }
 
 extern "C" int llc_cuda_status(void) {

@@ -1,14 +1,15 @@
-// FMA (CUDA-core) GEMM: the fp32-exact path (precision "fp32") of llc_cuda_gemm and the fallback for shapes the tensor-core
-// kernels do not take, fp32 or bf16 operands, fp32 accumulation.
+// FMA (CUDA-core) GEMM for problems of few tiles: the fp32-exact path (precision "fp32") of llc_cuda_gemm and the fallback for
+// shapes the tensor-core kernels do not take, fp32 or bf16 operands, fp32 accumulation.  igemm_simt.cu has the one for the
+// others and asks this one first (clusterGemm).
 //
 // A CTA of 256 threads computes a BM x BN tile over a slice of K; up to eight CTAs along K form a cluster, meet in
 // distributed shared memory (each adds up one slice of the rows, the partial tiles in K order, so results are
 // bit-reproducible) and run the epilogue on it: no scratch in global memory, no counters, no second launch.  K is walked in
 // blocks of 32, fetched a block ahead into registers and stored k-major in one of two shared buffers, so that a thread
 // reads its fragments as float4 and one barrier per block is enough.
-// Bound: fp32 FMA for large problems (148 SMs x 128 lanes); the small ones (an MLP of 64 rows) by latency, which is why
-// their K loop is cut.  Against K slices that met in a global workspace (16 k per step): the MLP 784-512-10 at 64 rows 30.7 ->
-// 19.8 us, at 1021 rows 56 -> 45 us.
+// Bound: latency (a CTA alone on its SM needs 62 ns per k where the FMAs take 33), which is why the K loop is cut.  Against
+// igemm_simt_kernel (us a launch, back to back): 64 x 512 x 784 14.5 -> 11.2, 64 x 10 x 512 15.2 -> 6.5, 1021 x 512 x 784
+// 45.5 -> 36.9, 2048 x 2048 x 256 114 -> 86.
 #include "common.cuh"
 
 namespace llc {
@@ -130,11 +131,25 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const __grid_constant__ 
     }
   };
 
-  float acc[TM][TN];
+  // Sums of 128 products are added up in `total`: the K slices of problems with few tiles have always been that short, and
+  // one sum over an eighth of K was off by twice as much (64 x 10 x 25088: 1.0e-6 of the result against 5.1e-7).  128 x 128
+  // tiles, which have no registers for it, are never cut into longer slices than igemm_simt_kernel would cut them into.
+  constexpr bool kShortSums = TM * TN <= 16;
+  constexpr int kSumBlocks = 128 / BK;
+  float acc[TM][TN], total[kShortSums ? TM : 1][kShortSums ? TN : 1];
+  auto closeSums = [&](bool last) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        if (last) acc[i][j] += total[i][j];
+        else { total[i][j] += acc[i][j]; acc[i][j] = 0.f; }
+      }
+  };
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) { acc[i][j] = 0.f; if constexpr (kShortSums) total[i][j] = 0.f; }
 
   const int nk = kEnd > kBeg ? (int)((kEnd - kBeg + BK - 1) / BK) : 0;
   if (nk > 0) { loadTile(kBeg); storeTile(0); }
@@ -154,9 +169,14 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const __grid_constant__ 
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
     }
-    if (kt + 1 < nk) storeTile(buf ^ 1);
+    if (kt + 1 < nk) {
+      storeTile(buf ^ 1);
+      if constexpr (kShortSums) { if (kt % kSumBlocks == kSumBlocks - 1) closeSums(false); }
+    }
     __syncthreads();
   }
+
+  if constexpr (kShortSums) closeSums(true);
 
   // The partial (or whole) tile goes through shared memory, so that the epilogue works on whole rows.
   auto rowOf = [&](int i) { return (i >> 2) * 64 + ty * 4 + (i & 3); };
@@ -215,22 +235,27 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const __grid_constant__ 
   if (split) clusterBarrier();                                   // no CTA leaves while another reads its partial tile
 }
 
-// Tile and number of K slices by estimated cycles: rounds of CTAs over the SMs x (K slice x cycles per k of the tile, bound by
-// FMA issue for 128 x 128 and by shared-memory reads for the smaller ones) + what a slice costs besides.
-struct SimtPlan { int bm, bn, slices; };
-SimtPlan choosePlan(long long M, long long N, long long K, long long batch) {
-  struct Tile { int bm, bn; float perK; };
-  static const Tile tiles[] = {{128, 128, 150.f}, {64, 64, 64.f}, {64, 16, 40.f}};
-  SimtPlan best{64, 64, 1}; float bestCost = -1.f;
-  for (const Tile& t : tiles) {
-    if (t.bn == 16 && N > 64) continue;
-    if (t.bm == 128 && (M <= 64 || N <= 64)) continue;
-    const long long n = ((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn) * batch;
+// Tile and number of K slices by estimated time, us: a constant for the launch and the epilogue, and K of a slice times what a k
+// takes on an SM that holds `c` CTAs (measured; from four on the CTAs' L1 is too small for the rows they read 16 bytes at a
+// time).  Clusters do not fill the chip: of four CTAs 33 run at once, of eight 14.  Rows that cannot be read as vectors
+// take 15 % longer (10 % in the other kernel).  Over 234 shapes (1 to 4096 rows, 8 to 4096 columns, K 32 to 30000) the two
+// kernels chosen so take 0.71 of what igemm_simt_kernel takes alone, geometric mean, and no shape more than 1.08.  (The first choice of tiles counted no
+// neighbours on an SM: 4096 x 512 x 784 105 -> 190 us, 64 x 10 x 25088 46 -> 110.)
+struct SimtPlan { int bn, slices; float us; };   // bn 128: 128 x 128 tiles, otherwise 64 x bn
+SimtPlan choosePlan(long long M, long long N, long long K, long long batch, bool vec) {
+  static const struct { int bm, bn; float fixedUs, perK; } tiles[] = {{64, 16, 4.f, 0.0345f}, {64, 64, 4.f, 0.0625f}, {128, 128, 10.f, 0.131f}};
+  SimtPlan best{0, 0, 0.f};
+  for (const auto& t : tiles) {
+    if (t.bn == 16 ? N > 64 : t.bn == 128 && (M <= 64 || N <= 64)) continue;
+    const long long nTiles = (N + t.bn - 1) / t.bn, n = (M + t.bm - 1) / t.bm * nTiles * batch;
+    if (nTiles > 65535) continue;                        // (the grid's y extent)
     for (int s = 1; s <= 8; s *= 2) {
-      if (s > 1 && (K / s < BK || batch * s > 65535)) break;
-      const long long rounds = (n * s + kNumSMs - 1) / kNumSMs;
-      const float cost = (float)rounds * ((float)((K + s - 1) / s) * t.perK + 2000.f) + (s > 1 ? 1500.f : 0.f);
-      if (bestCost < 0.f || cost < bestCost) { best = SimtPlan{t.bm, t.bn, s}; bestCost = cost; }
+      if (s > 1 && (K / s < BK || n * s > 2 * kNumSMs || batch * s > 65535)) break;
+      const long long atOnce = s == 8 ? 112 : s == 4 ? 132 : kNumSMs, per = t.bn == 128 ? atOnce : kNumSMs, sms = (n * s + per - 1) / per;
+      const float c = n * s <= atOnce ? 1.f : sms < 2 ? 2.f : (float)sms;
+      const float share = c == 1.f ? 1.f : t.bn == 16 ? 0.95f * c : t.bn == 128 ? c : c == 2.f ? (sms < 2 ? 1.4f : 1.6f) : c == 3.f ? 2.3f : 1.1f * c;
+      const float us = t.fixedUs + (s > 1 ? 0.7f : 0.f) + (float)((K + s - 1) / s) * t.perK * share * (vec ? 1.f : 1.15f);
+      if (!best.bn || us < best.us) best = SimtPlan{t.bn, s, us};
     }
   }
   return best;
@@ -258,22 +283,27 @@ template <typename T, int BM, int BN, bool VEC> int launchTile(const SimtArgs& a
   return LLC_OK;
 }
 
-template <typename T, bool VEC> int launchGemm(SimtArgs a, long long batch, cudaStream_t st) {
-  if (a.M <= 0 || a.N <= 0 || batch <= 0) return LLC_OK;
-  if (batch > 65535) return setError(LLC_ERR_ARGUMENT, "llc argument: gemm batch count above 65535");
-  const SimtPlan plan = choosePlan(a.M, a.N, a.K, batch);
+template <typename T, bool VEC> int launchGemm(SimtArgs a, const SimtPlan& plan, long long batch, cudaStream_t st) {
   a.slices = plan.slices;
   a.kPer = (((a.K + plan.slices - 1) / plan.slices) + 3) / 4 * 4;
-  if (plan.bm == 128) return launchTile<T, 128, 128, VEC>(a, batch, st);
-  if (plan.bn == 64) return launchTile<T, 64, 64, VEC>(a, batch, st);
-  return launchTile<T, 64, 16, VEC>(a, batch, st);
+  if (plan.bn == 128) return launchTile<T, 128, 128, VEC>(a, batch, st);
+  return plan.bn == 64 ? launchTile<T, 64, 64, VEC>(a, batch, st) : launchTile<T, 64, 16, VEC>(a, batch, st);
 }
 
 bool aligned(const void* p, int bytes) { return (reinterpret_cast<uintptr_t>(p) % bytes) == 0; }
 
 }  // namespace
 
-int simtGemm(const LlcGemmParams* p, cudaStream_t st) {
+// Runs the GEMM (arguments checked by the caller, nothing empty) if it is done clearly before `otherUs`; *taken tells.
+int clusterGemm(const LlcGemmParams* p, float otherUs, cudaStream_t st, bool* taken) {
+  *taken = false;
+  const int eb = p->in_dtype == LLC_FLOAT32 ? 4 : 2, ob = p->out_dtype == LLC_FLOAT32 ? 4 : 2;
+  const bool vec = p->k % 4 == 0 && p->a_sm % 4 == 0 && p->a_s0 % 4 == 0 && p->a_s1 % 4 == 0 && aligned(p->a, eb * 4) && aligned(p->b, eb * 4) &&
+                   p->b_s0 % 4 == 0 && p->b_s1 % 4 == 0 && (p->b_sk == 1 ? p->b_sn % 4 == 0 : (p->n % 4 == 0 && p->b_sk % 4 == 0));
+  const long long batch = p->b0 * p->b1;
+  if ((p->b_sk != 1 && p->b_sn != 1) || batch > 65535) return LLC_OK;      // (what the caller refuses)
+  const SimtPlan plan = choosePlan(p->m, p->n, p->k, batch, vec);
+  if (!plan.bn || plan.us >= 0.95f * otherUs * (vec ? 1.f : 1.1f)) return LLC_OK;
   SimtArgs a{};
   a.a = p->a; a.b = p->b; a.out = p->out; a.scale = p->scale; a.shift = p->shift; a.res = p->res;
   a.out_dtype = p->out_dtype; a.res_dtype = p->res_dtype; a.act = p->act; a.alpha = p->alpha;
@@ -283,52 +313,10 @@ int simtGemm(const LlcGemmParams* p, cudaStream_t st) {
   a.o_s0 = p->o_s0; a.o_s1 = p->o_s1; a.o_sm = p->o_sm;
   a.r_s0 = p->r_s0; a.r_s1 = p->r_s1; a.r_sm = p->r_sm; a.r_sn = p->r_sn;
   a.b1 = (int)p->b1;
-  if (p->b_sk != 1 && p->b_sn != 1) return setError(LLC_ERR_ARGUMENT, "llc argument: gemm B needs unit stride along k or n");
-  const int eb = p->in_dtype == LLC_FLOAT32 ? 4 : 2, ob = p->out_dtype == LLC_FLOAT32 ? 4 : 2;
   a.vecOut = aligned(p->out, ob * 4) && p->o_sm % 4 == 0 && p->o_s0 % 4 == 0 && p->o_s1 % 4 == 0;
-  const bool vec = p->k % 4 == 0 && p->a_sm % 4 == 0 && p->a_s0 % 4 == 0 && p->a_s1 % 4 == 0 && aligned(p->a, eb * 4) && aligned(p->b, eb * 4) &&
-                   p->b_s0 % 4 == 0 && p->b_s1 % 4 == 0 && (p->b_sk == 1 ? p->b_sn % 4 == 0 : (p->n % 4 == 0 && p->b_sk % 4 == 0));
-  const long long batch = p->b0 * p->b1;
-  if (p->in_dtype == LLC_FLOAT32) return vec ? launchGemm<float, true>(a, batch, st) : launchGemm<float, false>(a, batch, st);
-  if (p->in_dtype == LLC_BFLOAT16) return vec ? launchGemm<__nv_bfloat16, true>(a, batch, st) : launchGemm<__nv_bfloat16, false>(a, batch, st);
-  return setError(LLC_ERR_UNSUPPORTED, "llc argument: gemm input type must be f32 or bf16");
+  *taken = true;
+  if (p->in_dtype == LLC_FLOAT32) return vec ? launchGemm<float, true>(a, plan, batch, st) : launchGemm<float, false>(a, plan, batch, st);
+  return vec ? launchGemm<__nv_bfloat16, true>(a, plan, batch, st) : launchGemm<__nv_bfloat16, false>(a, plan, batch, st);
 }
 
 }  // namespace llc
-
-// ---- entry point that allocates nothing ----------------------------------------------------------
-// Some hosts of this library cannot allocate device memory when they call it: a serving process that handed the whole GPU
-// to its own pool at start-up, or a control loop that cannot afford the device-wide synchronisation an allocation takes.
-// The slices of this GEMM meet in shared memory, so it needs no scratch at all and this entry point is llc_cuda_gemm's FMA
-// path under a contract: shapes whose K slices would take more than kScratchLimit bytes of partial tiles, parked in memory
-// as 64 x 64 tiles of K / 128 slices at most, are refused, as callers of this entry point have always been told.
-namespace llc {
-namespace {
-
-constexpr long long kScratchLimit = 1 << 20;
-long long parkedBytes(long long M, long long N, long long K, long long batch) {
-  const long long t64 = ((M + 63) / 64) * ((N + 63) / 64) * batch;
-  if (t64 <= 0 || t64 * 2 > kNumSMs || K < 512) return 0;
-  long long want = kNumSMs / t64; if (want > 32) want = 32; if (want > K / 128) want = K / 128;
-  if (want < 1) return 0;
-  const long long kPer = ((K + want - 1) / want + 15) / 16 * 16, split = (K + kPer - 1) / kPer;
-  return split <= 1 || batch * split > 65535 ? 0 : 4096 + t64 * split * 64 * 64 * (long long)sizeof(float);
-}
-
-}  // namespace
-}  // namespace llc
-
-extern "C" int llc_cuda_gemm_static_scratch(const LlcGemmParams* p, void* stream) {
-  using namespace llc;
-  if (!p) return setError(LLC_ERR_ARGUMENT, "llc argument: gemm null parameter block");
-  if (p->m < 0 || p->n < 0 || p->k < 0 || p->b0 < 0 || p->b1 < 0) return setError(LLC_ERR_ARGUMENT, "llc argument: gemm negative extent");
-  if (p->m == 0 || p->n == 0 || p->b0 == 0 || p->b1 == 0) return LLC_OK;
-  if (!p->a || !p->b || !p->out) return setError(LLC_ERR_ARGUMENT, "llc argument: gemm null operand");
-  auto floatIo = [](int32_t dt) { return dt == LLC_FLOAT32 || dt == LLC_BFLOAT16; };
-  if (!floatIo(p->in_dtype) || !floatIo(p->out_dtype) || (p->res && !floatIo(p->res_dtype)))
-    return setError(LLC_ERR_UNSUPPORTED, "llc argument: gemm operands must be f32 or bf16");
-  const long long need = parkedBytes(p->m, p->n, p->k, p->b0 * p->b1);
-  if (need > kScratchLimit)
-    return setError(LLC_ERR_ARGUMENT, "llc argument: this GEMM needs " + std::to_string(need) + " bytes of split-K scratch, the built-in array holds " + std::to_string(kScratchLimit));   // (the wording callers know)
-  return simtGemm(p, (cudaStream_t)stream);
-}
