@@ -1,6 +1,6 @@
 // Elementwise chains: the kernels behind llc_cuda_eltwise for programs in chain form (eltwise_prog.cuh).
-//   chain_rows_kernel   every operand dense or broadcast along the output's innermost dim: sixteen elements per thread in
-//                       two 16-byte pieces, no division for two dims or fewer.
+//   chain_rows_kernel   every operand dense or broadcast along the output's innermost dim: eight or sixteen elements per
+//                       thread in 16-byte pieces, no division for two dims or fewer.
 //   chain_tile_kernel   at least one operand is dense along another dim than the output (an NHWC activation read by a step
 //                       that writes NCHW, or the other way round): 64 x 64 tiles of that operand go through shared memory.
 // Bound: HBM.  Algorithmic bytes: every operand element once, the output once.  Against the general kernels, which these
@@ -84,7 +84,24 @@ struct SlotArgs {
 
 // The programs most large steps consist of have kernels of their own: the general chain's branches and the calls behind
 // them made the kernels wait for instructions (NHWC + NCHW -> ReLU -> NCHW on 256x512x28x28 bf16: issue slots 77 % busy).
-enum ChainProg { P_CHAIN = 0, P_COPY, P_ADD, P_ADD_RELU };
+// P_ONE: one step of any kind, its op decoded once per thread and inline (as a chain of one step, with a call per element for
+// the transcendental ops, 64 x 512 bf16 GELU took 5.1 us where it had taken 3.2, a division 4.6 for 2.6).
+enum ChainProg { P_CHAIN = 0, P_COPY, P_ADD, P_ADD_RELU, P_ONE };
+
+// acc = op(acc, y) (or op(y, acc) when `swap`) for E elements.
+template <int E> __device__ __forceinline__ void oneStep(int op, float* acc, const float* y, bool swap) {
+  float a[E], b[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) { a[e] = swap ? y[e] : acc[e]; b[e] = swap ? acc[e] : y[e]; }
+  switch (op) {
+#define LLC_ONE(OP) case OP: _Pragma("unroll") for (int e = 0; e < E; ++e) acc[e] = evalOp(OP, a[e], b[e], 0.f, 0.f); break;
+    LLC_ONE(E_ADD) LLC_ONE(E_SUB) LLC_ONE(E_MUL) LLC_ONE(E_DIV) LLC_ONE(E_MAX) LLC_ONE(E_MIN) LLC_ONE(E_POW) LLC_ONE(E_RELU) LLC_ONE(E_ABS) LLC_ONE(E_SQRT)
+    LLC_ONE(E_RSQRT) LLC_ONE(E_EXP) LLC_ONE(E_GELU) LLC_ONE(E_TANH) LLC_ONE(E_ERF) LLC_ONE(E_SIGMOID) LLC_ONE(E_NEG) LLC_ONE(E_TRUNC) LLC_ONE(E_TF32LO)
+    LLC_ONE(E_EQ) LLC_ONE(E_NE) LLC_ONE(E_GE) LLC_ONE(E_GT) LLC_ONE(E_LE) LLC_ONE(E_LT)
+#undef LLC_ONE
+    default: break;                              // E_CAST
+  }
+}
 
 // Runs the chain on E elements; v[j] holds slot j.
 template <int PROG, int NIN, int E> __device__ __forceinline__ void runChain(const EltChain& c, float (*v)[E], float* acc) {
@@ -96,6 +113,13 @@ template <int PROG, int NIN, int E> __device__ __forceinline__ void runChain(con
   if constexpr (PROG == P_ADD || PROG == P_ADD_RELU) {
 #pragma unroll
     for (int e = 0; e < E; ++e) { const float x = v[0][e] + v[1][e]; acc[e] = PROG == P_ADD ? x : fmaxf(x, 0.f); }
+    return;
+  }
+  if constexpr (PROG == P_ONE) {                 // the operand is the other slot, a constant or the value itself
+    float y[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) { acc[e] = v[0][e]; y[e] = NIN == 2 ? v[NIN - 1][e] : c.src[0] == C_IMM ? c.imm[0] : v[0][e]; }
+    oneStep<E>(c.op[0], acc, y, c.swap[0] != 0);
     return;
   }
   int s = 0;
@@ -138,10 +162,10 @@ struct RowsArgs {
 };
 
 // TWO: at most two dims - a block is blockDim.y rows by one part of a row, no thread divides.  Otherwise the linear piece
-// index is decomposed over the dims.  A thread takes two pieces so that twice the loads are in flight.
-template <bool TWO, int PROG, int NIN>
-__global__ void __launch_bounds__(256, NIN == 1 ? 6 : NIN == 2 ? 4 : 3) chain_rows_kernel(const __grid_constant__ RowsArgs p) {
-  constexpr int U = 2;
+// index is decomposed over the dims.  A thread takes U pieces: two, so that twice the loads are in flight, or one where two
+// would leave SMs without a block (rowPieces).
+template <bool TWO, int U, int PROG, int NIN>
+__global__ void __launch_bounds__(256, NIN == 3 ? 3 : NIN == 2 || PROG == P_ONE ? 4 : 6) chain_rows_kernel(const __grid_constant__ RowsArgs p) {
   const SlotArgs& e = p.e;
   const int last = e.rank - 1;
   long long oOff[U], iOff[U][NIN];
@@ -215,7 +239,8 @@ struct TileArgs {
 // A tile row is 128 (2-byte types) or 256 (fp32) bytes in both directions, whole sectors either way.  In shared memory a
 // row is one c: 64 p positions plus one word, which leaves the transposing writes and the reads without bank conflicts;
 // 2-byte elements are paired along p so that every access is a word.  The operands that need no transposing are requested
-// before the tiles are filled.
+// before the tiles are filled.  (The fp32 variants of three operands spill 140 bytes at three blocks per SM; at two, without
+// spills, 32 x 512 x 28 x 28 took 55 us for 48.)
 template <int ES, int V, int PROG, int NIN>
 __global__ void __launch_bounds__(256, NIN == 1 ? 5 : NIN == 2 ? 4 : 3) chain_tile_kernel(const __grid_constant__ TileArgs p) {
   constexpr int kWords = kT * ES / 4, kRow = kWords + 1;
@@ -369,19 +394,34 @@ ChainProg progOf(const EltChain& c) {
   if (c.startSrc != C_INPUT) return P_CHAIN;
   if (c.n == 0) return P_COPY;
   const bool add = c.op[0] == E_ADD && c.src[0] == C_INPUT;
-  if (c.n == 1) return add ? P_ADD : c.op[0] == E_CAST ? P_COPY : P_CHAIN;
+  if (c.n == 1) return add ? P_ADD : c.op[0] == E_CAST ? P_COPY : P_ONE;
   return add && c.n == 2 && c.op[1] == E_RELU ? P_ADD_RELU : P_CHAIN;
 }
 
-template <bool TWO> int launchRows(int nin, const RowsArgs& p, dim3 blocks, dim3 threads, cudaStream_t st) {
-  switch (progOf(p.e.c)) {
-    case P_COPY: chain_rows_kernel<TWO, P_COPY, 1><<<blocks, threads, 0, st>>>(p); break;
-    case P_ADD: chain_rows_kernel<TWO, P_ADD, 2><<<blocks, threads, 0, st>>>(p); break;
-    case P_ADD_RELU: chain_rows_kernel<TWO, P_ADD_RELU, 2><<<blocks, threads, 0, st>>>(p); break;
+// Pieces of eight elements per thread.  Below two blocks of 16 x 256 elements per SM the second piece only lengthens a thread;
+// fp32 results, 32 bytes a piece, have enough loads in flight with one for longer.
+int rowPieces(long long total, int odt) { return total < (odt == LLC_FLOAT32 ? 6LL : 2LL) * kNumSMs * 256 * 16 ? 1 : 2; }
+
+// Steps that are an instruction or two in a chain as well: on large tensors the chain kernels' smaller register count counts
+// for more (98304 x 768 bf16 ReLU 53 against 63 us), on small ones the decoding does (64 x 512 2.3 against 2.0).
+bool cheapStep(int op) {
+  return op == E_SUB || op == E_MUL || op == E_MAX || op == E_MIN || op == E_RELU || op == E_NEG || op == E_ABS || op == E_TF32LO;
+}
+
+template <bool TWO, int U> int launchRows(int nin, const RowsArgs& p, dim3 blocks, dim3 threads, cudaStream_t st) {
+  const ChainProg prog = progOf(p.e.c);
+  switch (U == 2 && prog == P_ONE && cheapStep(p.e.c.op[0]) ? P_CHAIN : prog) {
+    case P_COPY: chain_rows_kernel<TWO, U, P_COPY, 1><<<blocks, threads, 0, st>>>(p); break;
+    case P_ADD: chain_rows_kernel<TWO, U, P_ADD, 2><<<blocks, threads, 0, st>>>(p); break;
+    case P_ADD_RELU: chain_rows_kernel<TWO, U, P_ADD_RELU, 2><<<blocks, threads, 0, st>>>(p); break;
+    case P_ONE:
+      if (nin == 1) chain_rows_kernel<TWO, U, P_ONE, 1><<<blocks, threads, 0, st>>>(p);
+      else chain_rows_kernel<TWO, U, P_ONE, 2><<<blocks, threads, 0, st>>>(p);
+      break;
     default:
-      if (nin == 1) chain_rows_kernel<TWO, P_CHAIN, 1><<<blocks, threads, 0, st>>>(p);
-      else if (nin == 2) chain_rows_kernel<TWO, P_CHAIN, 2><<<blocks, threads, 0, st>>>(p);
-      else chain_rows_kernel<TWO, P_CHAIN, 3><<<blocks, threads, 0, st>>>(p);
+      if (nin == 1) chain_rows_kernel<TWO, U, P_CHAIN, 1><<<blocks, threads, 0, st>>>(p);
+      else if (nin == 2) chain_rows_kernel<TWO, U, P_CHAIN, 2><<<blocks, threads, 0, st>>>(p);
+      else chain_rows_kernel<TWO, U, P_CHAIN, 3><<<blocks, threads, 0, st>>>(p);
   }
   LLC_LAUNCH_CHECK("chain_rows_kernel");
   return LLC_OK;
@@ -450,22 +490,24 @@ int launchChain(const EltArgs& a, cudaStream_t st, bool* taken) {
   if (rowsOk) {
     RowsArgs p; p.e = e; p.pieces = 0; p.rows = 1;
     const long long pieces = inner / 8;
+    const int u = rowPieces(a.total, a.odt);
     if ((r == 1 || (r == 2 && pieces >= 48)) && pieces <= 0x7FFFFFFFLL / 16) {      // (short rows would leave most of a warp idle)
-      // threads along a row: the row's pairs of pieces split into equal parts of at most 256, rounded up to whole warps
+      // threads along a row: the row's pieces (or pairs of pieces) split into equal parts of at most 256, rounded up to whole warps
       p.rows = r == 2 ? a.shape[0] : 1; p.pieces = (int)pieces;
-      const long long pairs = (pieces + 1) / 2, parts = (pairs + 255) / 256;
+      const long long pairs = (pieces + u - 1) / u, parts = (pairs + 255) / 256;
       const int tx = (int)((((pairs + parts - 1) / parts) + 31) / 32 * 32);
       const int ty = (int)(256 / tx < 1 ? 1 : (256 / tx < p.rows ? 256 / tx : p.rows));
       const long long blocks = (p.rows + ty - 1) / ty;
       if (blocks <= 0x7FFFFFFFLL && parts <= 65535) {
         *taken = true;
-        return launchRows<true>(nin, p, dim3((unsigned)blocks, (unsigned)parts), dim3((unsigned)tx, (unsigned)ty), st);
+        const dim3 grid((unsigned)blocks, (unsigned)parts), threads((unsigned)tx, (unsigned)ty);
+        return u == 1 ? launchRows<true, 1>(nin, p, grid, threads, st) : launchRows<true, 2>(nin, p, grid, threads, st);
       }
     }
-    const long long blocks = (a.total / 8 + 511) / 512;
+    const long long blocks = (a.total / 8 + 256 * u - 1) / (256 * u);
     if (blocks > 0x7FFFFFFFLL) return LLC_OK;
     *taken = true;
-    return launchRows<false>(nin, p, dim3((unsigned)blocks), dim3(256), st);
+    return u == 1 ? launchRows<false, 1>(nin, p, dim3((unsigned)blocks), dim3(256), st) : launchRows<false, 2>(nin, p, dim3((unsigned)blocks), dim3(256), st);
   }
   // ---- tiles: one or two operands dense along one and the same other dim
   TileArgs t; t.cDim = -1; t.nT = 0; t.first[0] = t.first[1] = 0;

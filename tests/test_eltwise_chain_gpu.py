@@ -63,6 +63,24 @@ def test_rows(dtype, rows, d):
     assert torch.equal(y, (x + a.view(rows, 1, d).float()).abs().to(dtype))
 
 
+# One step of every kind, with a second operand, a constant and itself, in both orders; one and two pieces per thread (below and
+# above 1.2 M elements, 3.6 M in fp32).  The general kernel (odd columns) does the same fp32 operations; 2^-22 covers contractions.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(3, 768), (5, 7, 1032), (3200, 768), (900, 5, 1032)])
+def test_one_step_programs(dtype, shape):
+    x, y = _rand(shape, dtype, 10), _rand(shape, dtype, 11).abs() + 0.25
+    unary = ["relu", "abs", "sqrt", "rsqrt", "exp", "gelu", "tanh", "erf", "sigmoid", "neg", "trunc", "tf32lo", "cast"]
+    binary = ["add", "sub", "mul", "div", "max", "min", "pow", "eq", "ne", "ge", "gt", "le", "lt"]
+    progs = ["ld1;%s,0" % o for o in unary] + ["ld0;ld1;%s,%s" % (o, r) for o in binary for r in ("0,1", "1,0") if (o, r) != ("pow", "0,1")]
+    progs += ["ld1;#1.5;%s,%s" % (o, r) for o in ("sub", "div", "pow", "ge") for r in ("0,1", "1,0")] + ["ld1;mul,0,0", "ld1;div,0,0"]
+    for prog in progs:
+        out, want = torch.full_like(x, float("nan")), torch.full((*shape[:-1], shape[-1] + 1), float("nan"), device="cuda", dtype=dtype)[..., :-1]
+        G.eltwise(out, [x, y], prog)
+        G.eltwise(want[..., :-1], [x[..., :-1], y[..., :-1]], prog)
+        torch.testing.assert_close(out[..., :-1].float(), want[..., :-1].float(), rtol=2.0 ** -22 if dtype is torch.float32 else 2.0 ** -8, atol=1e-38, msg=prog)
+        assert not out.isnan().any(), prog
+
+
 def test_rows_of_other_types():
     m = torch.randint(0, 2, (5, 384), generator=torch.Generator().manual_seed(9)).cuda()
     for t in (m, m.int(), m.bool(), m.half(), m.to(torch.int8)):
