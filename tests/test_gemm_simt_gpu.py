@@ -68,3 +68,23 @@ def test_k_slices_are_reproducible_and_streams_share_nothing():
             G.gemm(a, b, o)
     torch.cuda.synchronize()
     assert all(torch.equal(outs[0], o) for o in outs)
+
+
+def test_the_entry_point_with_its_own_array_at_a_long_k():
+    """64 x 10 x 8192 goes to the kernel whose K slices meet in that array; the second call finds what the first left there."""
+    from ctypes import byref, c_void_p
+
+    from llcompiler_b200 import _capi as C
+    m, n, k = 64, 10, 8192
+    a, b = torch.randn(1, 1, m, k, device="cuda"), torch.randn(1, 1, n, k, device="cuda")
+    want, mag = a.double() @ b.double().transpose(2, 3), a.double().abs() @ b.double().abs().transpose(2, 3)
+    for _ in range(2):
+        out = torch.full((1, 1, m, n), float("nan"), device="cuda")
+        p = C.LlcGemmParams()
+        p.a, p.b, p.out = (c_void_p(t.data_ptr()) for t in (a, b, out))
+        p.in_dtype = p.out_dtype = p.res_dtype = 4
+        p.precision, p.alpha, p.act = C.PREC["fp32"], 1.0, C.ACT["none"]
+        p.b0, p.b1, p.m, p.n, p.k, p.a_sm, p.b_sk, p.b_sn, p.o_sm = 1, 1, m, n, k, k, 1, k, n
+        C.check(C.lib().llc_cuda_gemm_static_scratch(byref(p), c_void_p(torch.cuda.current_stream().cuda_stream)))
+        torch.cuda.synchronize()
+        assert ((out.double() - want).abs() <= (k // 32 + 40) * 2.0 ** -24 * mag).all()      # 32 slices, summed in order
